@@ -104,13 +104,13 @@ def _config(case):
 
 def _weights(cfg, seed):
     """bf16 tensors by checkpoint name: matrices N(0, 0.64 / sqrt(input width)), which is the usual 0.02 at a width of 1024, norm
-    weights near one. Expert stacks are returned whole as well."""
+    weights near one, routers that prefer few experts clearly as trained ones do. Expert stacks are returned whole as well."""
     g = torch.Generator(device="cuda").manual_seed(seed)
     H, d, V = cfg.hidden_size, cfg.head_dim, cfg.vocab_size
 
 
-    def mat(*shape):
-        return torch.empty(*shape, dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.64 * shape[-1] ** -0.5, generator=g)
+    def mat(*shape, gain=0.64):
+        return torch.empty(*shape, dtype=torch.bfloat16, device="cuda").normal_(0.0, gain * shape[-1] ** -0.5, generator=g)
 
     def norm(n):
         return (1.0 + 0.1 * torch.randn(n, device="cuda", generator=g)).to(torch.bfloat16)
@@ -125,7 +125,7 @@ def _weights(cfg, seed):
             sd[p + f"self_attn.{n}_proj.weight"] = mat(rows, cols)
         if cfg.is_moe_layer(i):
             E, I = cfg.num_experts, cfg.moe_intermediate_size
-            sd[p + "mlp.gate.weight"] = mat(E, H)
+            sd[p + "mlp.gate.weight"] = mat(E, H, gain=3.0)
             gu, dn = mat(E, 2 * I, H), mat(E, H, I)
             stacks[i] = (gu, dn)
             for e in range(E):
