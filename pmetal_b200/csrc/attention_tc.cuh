@@ -49,8 +49,6 @@ __device__ __forceinline__ float fast_rcp(float x) {
   return y;
 }
 
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 // Store 32 bf16 (packed in pk[16]) of row r into a [128][128] bf16 tile made of two 128B-swizzled
 // [128][64] boxes; c = index of the 32-column chunk (0..3). This is the layout tcgen05.mma reads as a
 // K-major operand (rows = M/N) and, with the other descriptor, as an MN-major operand (rows = K).

@@ -31,9 +31,7 @@ struct GemmParams {
   int seg_end[4];
   int seg_r;
   int tmem_cols;
-  int kps;         // K blocks per pipeline stage (CTA-pair kernel)
-  int fwd_full;    // CTA-pair kernel: each CTA counts its own TMA bytes; the partner forwards one arrive per stage
-  int commit_both; // CTA-pair kernel: signal both CTAs' barriers with one commit
+  int group_m;     // CTA-pair kernel: row blocks per group of the tile order
   int* status;
   float* ws;             // out_mode 6: [tiles][splits][128][bn] fp32 partial tiles
   unsigned* ws_cnt;      // out_mode 6: [tiles][4] arrival counters, zero between launches

@@ -393,7 +393,6 @@ extern "C" int pm_gemm_q4_2sm(const void* A, int lda, int a_rows, const void* co
   p.seg_mode = seg_mode; p.seg_r = seg_r;
   for (int i = 0; i < 4; ++i) p.seg_end[i] = (seg_mode && seg_end) ? seg_end[i] : 0x7fffffff;
   p.status = status;
-  p.kps = 1; p.fwd_full = 1; p.commit_both = 0;
   int stages = (227 * 1024 - 2048) / kQ4StageBytes;
   if (stages > kMaxStages) stages = kMaxStages;
   p.stages = stages;

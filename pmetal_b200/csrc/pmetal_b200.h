@@ -184,7 +184,7 @@ int pm_gdn_scan(const float* q, const float* k, const float* v, const float* g, 
     float* y, int B, int T, int H, int dk, int dv, cudaStream_t st);
 
 // ---------------------------------------------------------------- gemm_2sm.cu
-// Same contract as pm_gemm_bf16 with the tile fixed at 256 x 256 per CTA pair.
+// Same contract as pm_gemm_bf16 with the tile 256 rows high per CTA pair; its width (256 or 128 columns) is chosen here.
 int pm_gemm_bf16_2sm(const void* A, int a_mn, int lda, int a_rows, const void* B, int b_mn, int ldb, int b_rows,
     const void* A2, int a2_mn, int lda2, int a2_k, const void* B2, int b2_mn, int ldb2, int b2_rows, void* D, int
     out_mode, int ldd, const void* R, int ldr, int M, int N, int K, int K2, int n_store, float alpha, int splits,

@@ -174,9 +174,9 @@ def _seg_ends(seg_sizes: Sequence[int]):
 def raw_gemm(A, a_mn, lda, a_rows, B, b_mn, ldb, b_rows, D, out_mode, ldd, M, N, K, *, A2=None, a2_mn=0, lda2=0,
              a2_k=0, B2=None, b2_mn=0, ldb2=0, b2_rows=0, K2=0, R=None, ldr=0, n_store=0, alpha=1.0, bn=128, splits=1,
              seg_mode=0, seg_sizes=(), seg_r=0, max_ctas=0, tail=None, tail_from=0) -> None:
-    """One GEMM launch; ``tail`` (fp32) takes the columns from ``tail_from`` on. 256-wide tiles on at least 256 rows go to the CTA-pair (cta_group::2) kernel."""
+    """One GEMM launch; ``tail`` (fp32) takes the columns from ``tail_from`` on. Wide tiles on at least 256 rows go to the CTA-pair (cta_group::2) kernel, which chooses their width."""
     segs = _seg_ends(seg_sizes) if seg_mode else None
-    if USE_2SM and bn == 256 and M >= 256 and (seg_mode != 2 or all(s % 256 == 0 for s in seg_sizes[:-1])):
+    if USE_2SM and bn >= 128 and M >= 256 and (seg_mode != 2 or all(s % 256 == 0 for s in seg_sizes[:-1])):
         rc = lib().pm_gemm_bf16_2sm(_p(A), c_int(a_mn), c_int(lda), c_int(a_rows), _p(B), c_int(b_mn), c_int(ldb),
                                     c_int(b_rows), _p(A2), c_int(a2_mn), c_int(lda2), c_int(a2_k), _p(B2),
                                     c_int(b2_mn), c_int(ldb2), c_int(b2_rows), _p(D), c_int(out_mode), c_int(ldd),

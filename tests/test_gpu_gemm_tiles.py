@@ -1,0 +1,45 @@
+"""The CTA-pair GEMM at the edges of its tiles, of its staged epilogue and of its tile order."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(*shape, scale=1.0):
+    return (torch.randn(*shape, device="cuda") * scale).to(torch.bfloat16)
+
+
+def _near(y, ref, what):
+    """bf16 rounds to 2^-9 of a value; the fp32 sums of up to 9728 products of unit size in all stay within 1e-3."""
+    err = (y.float() - ref).abs()
+    assert bool((err <= ref.abs() * 2.0 ** -8 + 1e-3).all()), f"{what}: {float(err.max())}"
+
+
+# last row block of 1 .. 255 rows, columns that end inside a 64-wide piece, one and many groups of 16 row blocks (the last
+# one short), one k block and many, both tile widths, LoRA segments that end on multiples of 128 but not of 256
+@pytest.mark.parametrize("M,N,K,segs", [(256, 256, 64, ()), (257, 264, 72, ()), (511, 1000, 1024, ()), (4865, 1024, 136, ()),
+                                        (2048, 1024, 2048, (1024,)), (1300, 640, 320, (256, 128, 256)), (8193, 512, 200, (256, 256)),
+                                        (300, 4096, 9728, (2048, 1024, 1024))])
+def test_pair_gemm_tile_edges(M, N, K, segs):
+    from pmetal_b200.ops import native as nat
+    torch.manual_seed(M + N)
+    x, w, res = _rand(M, K), _rand(N, K, scale=K ** -0.5), _rand(M, N)
+    ref = x.float() @ w.float().t()
+    _near(nat.gemm(x, w), ref, "plain")
+    # the residual lives in a wider matrix, the result goes into one: neither may be written beside its columns
+    wide, out = _rand(M, N + 64), torch.full((M, N + 64), 7.0, dtype=torch.bfloat16, device="cuda")
+    nat.gemm(x, w, alpha=0.5, residual=wide[:, 8:N + 8], out=out[:, 16:N + 16])
+    _near(out[:, 16:N + 16], 0.5 * ref + wide[:, 8:N + 8].float(), "strided residual and result")
+    assert bool((out[:, :16] == 7).all()) and bool((out[:, N + 16:] == 7).all())
+    same = res.clone()
+    nat.gemm(x, w, residual=same, out=same)
+    _near(same, ref + res.float(), "residual in place")
+    if segs:
+        a, b = _rand(16 * len(segs), K, scale=K ** -0.5), _rand(N, 16, scale=0.2)
+        t = nat.lora_t(x, a, 2.0)
+        want, at = ref + res.float(), 0
+        for i, n in enumerate(segs):
+            want[:, at:at + n] += t[:, 16 * i:16 * i + 16].float() @ b[at:at + n].float().t()
+            at += n
+        _near(nat.gemm_lora(x, w, t, b, segs, 16, res), want, "segments")
+    nat.check_status()
