@@ -33,6 +33,10 @@ struct FaParams {
   const float* sink;
   const __nv_bfloat16* gate;
   long long ldg;
+  // forward kernel on a paged cache only: new tokens of n_seq sequences, keys behind a block table (64 tokens a block). A tile holds
+  // 128 >> rep_log2 tokens times the query heads of one kv head; q_tiles such tiles cover the longest sequence's new tokens.
+  const int *block_table, *seq_lens, *q_start, *q_lens;
+  int n_seq, max_blocks, q_tiles, rep_log2;
 };
 
 // 2^x on the SFU; -inf gives 0
@@ -70,5 +74,28 @@ __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t tile_addr, int s) {
   return make_smem_desc(tile_addr + s * 2048, static_cast<uint32_t>(kFaBox), 1024u);
 }
 
+// D (+)= A B over one tile: 8 MMAs of 16 elements of the reduction dimension each, operands [128][128] bf16 tiles (two boxes), read K-major
+// or MN-major. Called by a whole warp with warp-uniform arguments and issued by its elected lane: descriptors then are sums of two
+// uniform values, where a branch on the lane number makes the compiler treat each of them as divergent (about 1000 cycles for every
+// 8 MMAs, twice what the MMAs take).
+template <bool kAMn, bool kBMn>
+__device__ __forceinline__ void umma_tile(bool elected, uint32_t d_tmem, uint32_t a_addr, uint32_t b_addr, uint32_t idesc,
+                                          uint32_t accumulate) {
+  const uint64_t da = make_smem_desc(a_addr, kAMn ? static_cast<uint32_t>(kFaBox) : 16u, 1024u);
+  const uint64_t db = make_smem_desc(b_addr, kBMn ? static_cast<uint32_t>(kFaBox) : 16u, 1024u);
+  if (elected) {
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const uint32_t kmaj = (s >> 2) * (kFaBox >> 4) + (s & 3) * 2, mn = s * 128;      // units of 16 bytes
+      umma_f16(d_tmem, da + (kAMn ? mn : kmaj), db + (kBMn ? mn : kmaj), idesc, s > 0 ? 1u : accumulate);
+    }
+  }
+}
+
+// One [128][128] tile as two TMA boxes.
+__device__ __forceinline__ void tma_load_tile(uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int col, int row) {
+  tma_load_2d(dst, map, bar, col, row);
+  tma_load_2d(dst + kFaBox, map, bar, col + 64, row);
+}
 
 }  // namespace pm

@@ -394,9 +394,6 @@ static int launch_pair(GemmParams p, const void* A, int lda, int a_rows, const v
 // 128 columns takes about 0.65 of one of 256 (it moves three quarters of the bytes), and a tile about 4 blocks' time more
 // than its blocks. LoRA segments must end on tile boundaries.
 static int pair_width(const GemmParams& p, int pairs) {
-#ifdef PM_FORCE_BN
-  return PM_FORCE_BN;
-#endif
   if (p.seg_mode == 1)
     for (int i = 0; i < 3; ++i)
       if (p.seg_end[i] != 0x7fffffff && p.seg_end[i] % 256) return 128;

@@ -178,6 +178,21 @@ static inline int make_map(CUtensorMap* map, const void* ptr, uint64_t inner, ui
   return r == CUDA_SUCCESS ? 0 : -static_cast<int>(r) - 1000;
 }
 
+// The same with a middle dimension: [outer][mid][inner], strides in elements, box [box_outer][box_mid][box_inner].
+static inline int make_map3(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t mid, uint64_t outer, uint64_t ld_mid,
+                            uint64_t ld_outer, uint32_t box_inner, uint32_t box_mid, uint32_t box_outer) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc) return -1;
+  cuuint64_t dims[3] = {inner, mid, outer};
+  cuuint64_t strides[2] = {ld_mid * 2, ld_outer * 2};
+  cuuint32_t box[3] = {box_inner, box_mid, box_outer};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -static_cast<int>(r) - 1000;
+}
+
 static inline int operand_map(CUtensorMap* map, const void* ptr, int mn_major, int rows_total, int k_total, int ld,
                        int tile_rows) {
   if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (ld % 8)) return -2;

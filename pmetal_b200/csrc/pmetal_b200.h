@@ -55,6 +55,12 @@ int pm_paged_attn_static_max_rows(void);
 const char* pm_paged_attn_static_strerror(int code);
 
 // ---------------------------------------------------------------- attention_tc.cu
+// Causal attention of new tokens over a paged bf16 cache (blocks of 64 tokens, head_dim 128). q, out: [total_q, hq, 128] contiguous;
+// k_cache, v_cache: [num_blocks, 64, hkv, 128]; hq / hkv a power of two up to 128. Token i of sequence s (q_lens[s] new tokens from row
+// q_start[s], seq_lens[s] keys with them) sees the keys j <= seq_lens[s] - q_lens[s] + i. max_q: most new tokens of a sequence.
+int pm_paged_attn_tc(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
+    const int* seq_lens, const int* q_start, const int* q_lens, int num_seqs, int max_blocks, int num_blocks, int
+    total_q, int max_q, int hq, int hkv, float scale, int* status, cudaStream_t st);
 int pm_attn_fwd_tc_rect(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long
     long v_stride, void* out, long long o_stride, float* lse, const int* seq_start, int T, int Tk, int shift, int
     hq, int hkv, float scale, int* status, cudaStream_t st);

@@ -1,0 +1,82 @@
+"""Tile edges of the tcgen05 attention kernels: the packed forward / backward and the paged forward against fp32 PyTorch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return float((a.float() - b.float()).norm() / b.float().norm())
+
+
+def _dense(q, k, v, first, limit, scale):
+    """fp32 attention of q [T, hq, d]: query i sees the keys first[i] .. limit[i]."""
+    rep = q.shape[1] // k.shape[1]
+    kk, vv = (t.float().repeat_interleave(rep, 1).transpose(0, 1) for t in (k, v))
+    s = q.float().transpose(0, 1) @ kk.transpose(1, 2) * scale
+    j = torch.arange(k.shape[0], device=q.device)[None]
+    s = s.masked_fill(~((j >= first[:, None]) & (j <= limit[:, None])), float("-inf"))
+    return (s.softmax(-1) @ vv).transpose(0, 1)
+
+
+# (kv lengths, new tokens): one token beside a prompt, ends on and beside the 64-token block and the 128-row tile, an odd number of blocks
+PAGED = [([1, 130], [1, 130]), ([64, 65, 63], [64, 65, 63]), ([129, 700, 256], [128, 1, 200]), ([1000], [333]), ([127, 128, 129, 193], [100, 128, 129, 65])]
+
+
+@pytest.mark.parametrize("hq,hkv", [(4, 4), (8, 4), (16, 4), (8, 1)])
+@pytest.mark.parametrize("lens,qlens", PAGED)
+def test_paged_prompt_attention(hq, hkv, lens, qlens):
+    from pmetal_b200.models.kv_cache import PagedKVCache
+    from pmetal_b200.ops import native as nat
+    g = torch.Generator(device="cuda").manual_seed(sum(lens) + hq)
+    cache = PagedKVCache(1, hkv, 128, 48)
+    cache.free = [b for b in torch.randperm(48, generator=torch.Generator().manual_seed(3)).tolist()]
+    for t in (cache.k[0], cache.v[0]):
+        t.copy_(torch.randn(t.shape, device="cuda", generator=g))
+    for i, (n, m) in enumerate(zip(lens, qlens)):
+        cache.add_sequence(i)
+        if n > m:
+            cache.reserve(i, n - m)
+    meta = cache.prepare(list(range(len(lens))), qlens)
+    q = torch.randn(sum(qlens), hq, 128, device="cuda", generator=g).to(torch.bfloat16)
+    out = torch.full_like(q, float("nan"))
+    rc = nat.lib().pm_paged_attn_tc(nat._p(q), nat._p(cache.k[0]), nat._p(cache.v[0]), nat._p(out), nat._p(meta.block_table),
+                                    nat._p(meta.seq_lens), nat._p(meta.q_start), nat._p(meta.q_lens), nat.c_int(len(lens)),
+                                    nat.c_int(meta.block_table.shape[1]), nat.c_int(48), nat.c_int(sum(qlens)), nat.c_int(max(qlens)),
+                                    nat.c_int(hq), nat.c_int(hkv), nat.c_float(128 ** -0.5), nat._p(nat.status_word(q.device)), nat._stream())
+    assert rc == 0
+    at = 0
+    for i, (n, m) in enumerate(zip(lens, qlens)):
+        k, v = cache.gather(0, i)
+        lim = torch.arange(n - m, n, device="cuda")
+        want = _dense(q[at:at + m], k, v, torch.zeros_like(lim), lim, 128 ** -0.5)
+        # bf16 probabilities and outputs: 2^-9 each, relative to the row
+        assert _rel(out[at:at + m], want) < 6e-3, (i, n, m)
+        at += m
+    nat.check_status()
+
+
+def test_paged_dispatch_keeps_small_steps_on_the_split_kernel():
+    from pmetal_b200.ops.native import _paged_on_tensor_cores as tc
+    assert tc(1, 2048, 2048, 16, 8) and tc(6, 700, 700, 16, 8) and tc(1, 512, 12000, 16, 8)
+    assert not tc(64, 1, 8000, 16, 8) and not tc(1, 37, 37, 16, 8) and not tc(1, 128, 12000, 16, 8) and not tc(1, 2048, 2048, 12, 4)
+
+
+@pytest.mark.parametrize("lens", [[1, 127, 1, 128, 200], [300], [129, 64, 1, 1, 400, 55], [513]])
+@pytest.mark.parametrize("hq,hkv", [(4, 4), (8, 2)])
+def test_packed_attention_at_tile_edges(lens, hq, hkv):
+    from pmetal_b200.ops import functional as ops
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    T = sum(lens)
+    q, k, v = (torch.randn(T, h, 128, device="cuda", generator=g).to(torch.bfloat16).requires_grad_(True) for h in (hq, hkv, hkv))
+    start = torch.repeat_interleave(torch.tensor([sum(lens[:i]) for i in range(len(lens))]), torch.tensor(lens)).int().cuda()
+    w = torch.randn(T, hq, 128, device="cuda", generator=g)
+    o = ops._AttnCoreFn.apply(q, k, v, start, 128 ** -0.5, 0)
+    grads = torch.autograd.grad((o.float() * w).sum(), (q, k, v))
+    qf, kf, vf = (t.detach().float().requires_grad_(True) for t in (q, k, v))
+    want = _dense(qf, kf, vf, start.long(), torch.arange(T, device="cuda"), 128 ** -0.5)
+    ref = torch.autograd.grad((want * w.to(torch.bfloat16).float()).sum(), (qf, kf, vf))
+    assert _rel(o, want) < 6e-3
+    # bf16 P, dS, O and dO enter the products: a handful of 2^-9 roundings
+    for a, b in zip(grads, ref):
+        assert _rel(a, b) < 1.5e-2
