@@ -2,27 +2,21 @@
 
     python -m pmetal_b200.bench.decode_trace [--tokens 6]             one sequence, a few greedy tokens, no CUDA graphs
                                                                        (launch lists under a profiler)
-    python -m pmetal_b200.bench.decode_trace --phases [--batch 1]     per-phase device timestamps of the whole-step
-                                                                       decode kernel (csrc/decode_mega.cu): staging,
-                                                                       mat-vec, attention and barrier time per layer
+    python -m pmetal_b200.bench.decode_trace --phases [--batch 1]     device time of every kernel of a decode step, as the
+                                                                       profiler's activity records give it
 """
 import argparse
 import json
 import os
 
-PHASES = ["P1 stage", "P1 qkv mat-vec", "P1 barrier", "P2 attention", "P2 barrier", "P3 stage", "P3 o-proj mat-vec",
-          "P3 barrier", "P4 stage", "P4 gate/up mat-vec", "P4 barrier", "P5 stage", "P5 down mat-vec", "P5 barrier"]
-
 
 def phase_trace(model, batch: int, prompt_len: int = 128) -> dict:
-    """Median duration (us) of every phase over the layers of one decode step, read from the timestamps that CTA 0
-    writes when the kernel is given a trace buffer."""
+    """Median duration (us) and launches per step of every kernel of a decode step, and the span of a whole step. Chained kernels
+    start before their predecessor has ended, so the durations overlap."""
     import torch
+    from torch.profiler import ProfilerActivity, profile
 
     from ..models.generation import Generator
-    from ..ops import native
-    n_layers = len(model.layers)
-    dev = model.embed_tokens.device
     gen = Generator(model, num_blocks=1024, cuda_graphs=False)
     g = torch.Generator().manual_seed(5)
     prompts = [torch.randint(0, model.cfg.vocab_size, (prompt_len,), generator=g).tolist() for _ in range(batch)]
@@ -30,27 +24,19 @@ def phase_trace(model, batch: int, prompt_len: int = 128) -> dict:
     ids = gen.prefill(seqs, prompts).argmax(-1)
     for _ in range(3):
         ids = gen.decode_step(seqs, ids).argmax(-1)
-    trace = torch.zeros(n_layers * 16, dtype=torch.int64, device=dev)
-    make = native.decode_scratch
-
-    def with_trace(*a, **k):
-        d = make(*a, **k)
-        d["trace"] = trace
-        return d
-    native.decode_scratch = with_trace
-    model._mega_scratch.clear()
-    try:
-        for _ in range(3):
+    steps = 3
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        for _ in range(steps):
             ids = gen.decode_step(seqs, ids).argmax(-1)
         torch.cuda.synchronize()
-    finally:
-        native.decode_scratch = make
-        model._mega_scratch.clear()
-    t = trace.view(n_layers, 16).cpu()
-    d = (t[:, 1:15] - t[:, 0:14]).float()
-    out = {name: round(d[2:, i].median().item() / 1e3, 2) for i, name in enumerate(PHASES)}
-    out["layer_us"] = round(float((t[2:, 14] - t[2:, 0]).float().median()) / 1e3, 2)
-    out["all_layers_ms"] = round(float(t[-1, 14] - t[0, 0]) / 1e6, 3)
+    times = {}
+    events = [e for e in prof.events() if str(e.device_type).endswith("CUDA")]
+    for e in events:
+        name = e.name.split("(")[0].removeprefix("void ")
+        times.setdefault(name, []).append(e.time_range.elapsed_us())
+    out = {n: {"us": round(sorted(t)[len(t) // 2], 2), "per_step": round(len(t) / steps, 2)} for n, t in times.items()}
+    out["step_us"] = round((max(e.time_range.end for e in events) - min(e.time_range.start for e in events)) / steps, 1)
     return out
 
 

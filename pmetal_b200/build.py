@@ -26,15 +26,15 @@ CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-pthread"]   # 
 
 # sources (csrc/*.cu) that a product entry point can be built from alone, for a checkout where nothing is compiled yet
 COMPONENTS = {
-    "duvivik": ("attention_tc", "gemm_2sm", "gemm_tcgen05", "gemv", "latent_attn", "postnorm", "ssd_chunk", "ssm"),
-    "resevik": ("gemm_2sm", "gemm_tcgen05", "gemv", "grouped_gemm", "linear_attn", "moe_experts", "moe_quant", "postnorm",
+    "duvivik": ("attention_tc", "gemm_2sm", "gemm_skinny", "gemm_tcgen05", "gemv", "latent_attn", "postnorm", "ssd_chunk", "ssm"),
+    "resevik": ("gemm_2sm", "gemm_skinny", "gemm_tcgen05", "gemv", "grouped_gemm", "linear_attn", "moe_experts", "moe_quant", "postnorm",
                 "ssd_chunk", "window_attn"),
-    "vosezen": ("attention_tc", "gemm_2sm", "gemm_tcgen05", "gemv", "grouped_gemm", "latent_attn", "moe_experts", "moe_quant",
+    "vosezen": ("attention_tc", "gemm_2sm", "gemm_skinny", "gemm_tcgen05", "gemv", "grouped_gemm", "latent_attn", "moe_experts", "moe_quant",
                 "postnorm", "window_attn"),
-    "ravapel": ("attention_tc", "gated_linear", "gemm_2sm", "gemm_tcgen05", "gemv", "linear_attn", "postnorm", "sandwich", "ssd_chunk",
+    "ravapel": ("attention_tc", "gated_linear", "gemm_2sm", "gemm_skinny", "gemm_tcgen05", "gemv", "linear_attn", "postnorm", "sandwich", "ssd_chunk",
                 "window_attn"),
-    "decoder": ("attention", "attention_tc", "decode_mega", "elementwise", "gemm_2sm", "gemm_tcgen05", "gemv",
-                "grouped_gemm", "moe_quant"),
+    "decoder": ("attention", "attention_tc", "elementwise", "gemm_2sm", "gemm_skinny", "gemm_tcgen05", "gemv", "grouped_gemm",
+                "layer_stack", "moe_quant"),
 }
 
 

@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_row_kernel(const __nv_bfloat1
                                                               __nv_bfloat16* __restrict__ y,
                                                               __nv_bfloat16* __restrict__ h_out, float* __restrict__ rstd,
                                                               int H, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[8];
   const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const size_t base = static_cast<size_t>(row) * H;
@@ -998,11 +1000,10 @@ extern "C" int pm_rmsnorm_fwd(const void* x, const void* res, const void* w, voi
                               int H, float eps, cudaStream_t st) {
   if (H % 8) return -1;
   if (T <= 592 && H <= 4096) {        // fewer row groups than SMs: spread the rows instead
-    rmsnorm_fwd_row_kernel<<<T, 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(res),
-        static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y), static_cast<__nv_bfloat16*>(h_out), rstd, H,
-        eps);
-    return PM_LAUNCH_CHECK();
+    return static_cast<int>(launch_pdl(
+        rmsnorm_fwd_row_kernel, dim3(static_cast<unsigned>(T)), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(x),
+        static_cast<const __nv_bfloat16*>(res), static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
+        static_cast<__nv_bfloat16*>(h_out), rstd, H, eps));
   }
   rmsnorm_fwd_kernel<<<(T + 7) / 8, 256, 0, st>>>(
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(res),

@@ -3,8 +3,8 @@
 // be independent of the predecessor's output (reading weights, prefetching them into L2); pdl_wait() returns once the
 // predecessor has completed and its writes are visible. Every kernel of a chain calls pdl_launch_dependents() at its
 // top so that its successor can be scheduled as soon as all of this kernel's CTAs are resident. Both instructions are
-// no-ops in a kernel launched the ordinary way. The launch attribute is off unless PMETAL_PDL=1: inside captured CUDA
-// graphs the decode step measured about 8 % slower with it (1.40 ms against 1.31 ms per token on one B200).
+// no-ops in a kernel launched the ordinary way. launch_pdl sets the launch attribute inside a PdlScope (the chains of
+// layer_stack.cu) or with PMETAL_PDL=1.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdlib.h>
@@ -28,6 +28,15 @@ inline bool pdl_enabled() {
   return v != 0;
 }
 
+// While one is alive, launch_pdl calls of this thread carry the attribute.
+inline thread_local int pdl_scope_depth = 0;
+struct PdlScope {
+  const int on;
+  explicit PdlScope(bool enable) : on(enable ? 1 : 0) { pdl_scope_depth += on; }
+  ~PdlScope() { pdl_scope_depth -= on; }
+  PdlScope(const PdlScope&) = delete;
+};
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg{};
@@ -39,7 +48,7 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = pdl_scope_depth > 0 || pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

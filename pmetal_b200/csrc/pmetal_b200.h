@@ -91,17 +91,6 @@ int pm_attn_bwd_tc(const void* dout, long long do_stride, const void* q, long lo
     dq_stride, void* dk, long long dk_stride, void* dv, long long dv_stride, const int* seq_start, int T, int hq,
     int hkv, float scale, int* status, cudaStream_t st);
 
-// ---------------------------------------------------------------- decode_mega.cu
-// 1 when one launch can run the step: up to 16 rows, 1 / 2 / 4 query heads per kv head, reduction sizes that are
-// multiples of 32, and the staged activations fit in shared memory.
-int pm_decode_layers_supported(int M, int H, int hq, int hkv, int I);
-// layers: device array of n_layers DmLayer records (10 pointers each). bar: 2 words, counters: M * hkv words, all zero
-// at launch (a completed launch leaves the counters zero; the caller clears bar before every launch).
-int pm_decode_layers(const void* layers, int n_layers, int M, int H, int hq, int hkv, int I, float eps, float
-    scale, void* x, void* h, void* qkv, void* attn, void* act, float* part_o, float* part_ml, unsigned* counters,
-    const float* cs, const float* sn, const int* block_table, const int* seq_lens, const long long* slots, int
-    max_blocks, int n_split, unsigned* bar, int* status, unsigned long long* trace, cudaStream_t st);
-
 // ---------------------------------------------------------------- dp_fused.cu
 // ptr arrays hold `world` device addresses each (peer-mapped). shadows may be null.
 int pm_dp_reduce_adamw(const unsigned long long* grads, const unsigned long long* params, const unsigned long long*
@@ -209,6 +198,14 @@ int pm_gemm_q4_2sm(const void* A, int lda, int a_rows, const void* codes, const 
     int ldr, int M, int K2, int n_store, float alpha, int seg_mode, const int* seg_end, int seg_r, int max_ctas,
     int* status, cudaStream_t stream);
 
+// ---------------------------------------------------------------- gemm_skinny.cu
+// x: [M, K] rows ldx apart, w: [N, K] (swiglu: [2 N, K], gate rows first) rows ldw apart, y / res: [M, N] rows ldy / ldr apart (res
+// nullable, may be y). M <= 128; K, N and the row strides multiples of 8, pointers 16-byte aligned. splits 0: chosen here. chain: see
+// the head of this file. Returns a negative value for arguments outside of that.
+int pm_linear_skinny(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy, const
+    void* res, long long ldr, int M, int N, int K, int swiglu, float alpha, int splits, int chain, int* status,
+    cudaStream_t st);
+
 // ---------------------------------------------------------------- gemm_tcgen05.cu
 // Returns 0 on success, negative on argument / descriptor errors, or the CUDA error code.
 //   a_rows/b_rows: extent of the operand along M / N as seen by the tensor map (rows beyond it read as zero).
@@ -283,6 +280,18 @@ int pm_latent_assemble(const void* qd, long long ldq, int n_q, const void* kv, l
     v128, cudaStream_t st);
 // out [n, ldo] (H * dv columns) = the first dv channels of every head of o128 [n, H, 128].
 int pm_latent_take(const void* o128, int n, int H, int dv, void* out, long long ldo, cudaStream_t st);
+
+// ---------------------------------------------------------------- layer_stack.cu
+// Bytes of scratch that pm_layer_stack needs for T tokens.
+long long pm_layer_stack_scratch(int T, int H, int hq, int hkv, int I, int n_split);
+// layers: n_layers rows of 12 pointers on the host: input norm, q|k|v weight, q norm, k norm (0: none), output weight, post norm,
+// gate|up weight, down weight, key cache, value cache, key scales, value scales (0: bf16 cache, else int8). x: [T, H]; out: [T, H].
+// tensor_cores 1: attention through pm_paged_attn_tc, else pm_paged_attn_ex with n_split. Returns the first launcher's error.
+int pm_layer_stack(const long long* layers, int n_layers, const void* x, void* out, void* scratch, long long
+    scratch_bytes, int T, int H, int hq, int hkv, int I, float eps, float scale, const float* cs, const float* sn,
+    const long long* slots, const int* block_table, const int* seq_lens, const int* q_start, const int* q_lens, int
+    num_seqs, int max_blocks, int num_blocks, int max_q, int tensor_cores, int n_split, int* status, cudaStream_t
+    st);
 
 // ---------------------------------------------------------------- linear_attn.cu
 // Token-by-token recurrence. u [tokens, ldu]; cs / sn fp32 [tokens, R / 2] (unused when R is 0); rot: 1 pairs (i, i + R / 2),

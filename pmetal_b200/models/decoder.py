@@ -31,7 +31,6 @@ ALL_PROJ = ATTN_PROJ + MLP_PROJ
 
 
 # rows up to which linear layers run on the bandwidth-bound mat-vec kernel instead of tensor-core tiles (decode)
-DECODE_MEGA = os.environ.get("PMETAL_DECODE_MEGA", "1") == "1"
 GEMV_MAX_ROWS = int(os.environ.get("PMETAL_GEMV_MAX_ROWS", "16"))
 
 
@@ -406,19 +405,12 @@ class DecoderLM(nn.Module):
         T = x.shape[0]
         skinny = native and T <= GEMV_MAX_ROWS
         layers = self.layers
-        plain_cache = cache.quant is None and cache.window == 0      # bf16 blocks, nothing recycled
-        if (skinny and DECODE_MEGA and plain_cache and meta.max_q == 1 and T == meta.block_table.shape[0]
-                and self._mega_ok(T)):
-            # every layer of the step in one cooperative launch (csrc/decode_mega.cu)
+        addresses = self._stack_addresses(cache) if native else None
+        if addresses is not None:
+            # dense layers without adapters: all of them in one call of the runtime (csrc/layer_stack.cu)
             from ..ops import native as nat
-            table = self._mega_table(cache)
-            ns = nat.decode_splits(T, hkv, meta.max_kv)
-            sc = self._mega_scratch.get((T, ns))
-            if sc is None:
-                sc = self._mega_scratch[(T, ns)] = nat.decode_scratch(T, cfg.hidden_size, hq, hkv, cfg.intermediate_size,
-                                                                      ns, x.device)
-            x = nat.decode_layers(table, len(self.layers), x.contiguous(), sc, rope[0], rope[1], meta, hq, hkv,
-                                  cfg.intermediate_size, cfg.rms_norm_eps, d ** -0.5)
+            x = nat.layer_stack(addresses, x.contiguous(), meta, rope[0], rope[1], hq, hkv, cfg.intermediate_size, cache.num_blocks,
+                                cfg.rms_norm_eps, d ** -0.5)
             layers = ()
         for li, layer in enumerate(layers):
             at = layer.self_attn
@@ -514,56 +506,38 @@ class DecoderLM(nn.Module):
         from ..parallel.tp_model import moe_local_forward
         return moe_local_forward(layer.mlp, n2, h)
 
-    def _mega_ok(self, T: int) -> bool:
-        """The whole-step kernel covers dense layers with plain bf16 weights: no adapters, biases, sliding windows or
-        soft-capping."""
-        if not hasattr(self, "_mega_scratch"):
-            self._mega_scratch = {}
-            self._mega_tables = {}
+    def _stack_addresses(self, cache) -> Optional[List[int]]:
+        """Device addresses of every layer in the order of ``pm_layer_stack``, or None where a layer is not a dense one with plain
+        bf16 weights (adapters, packed weights, biases, experts, sliding windows, sharding) or the cache is not a bf16 or int8 one.
+        Looked up on every call: adapters and packed weights come and go."""
         cfg = self.cfg
-        ok = cfg.attn_logit_softcap <= 0 and cfg.head_dim == 128 and getattr(self, "tp_world", 1) == 1
-        if ok:            # checked on every call: adapters or packed weights may have been attached since the last one
-            for layer in self.layers:
-                at = layer.self_attn
-                if not isinstance(layer.mlp, MLP) or at.window:
-                    ok = False
-                    break
-                for lin in (at.qkv_proj, at.o_proj, layer.mlp.gate_up_proj, layer.mlp.down_proj):
-                    if (lin.lora_a is not None or getattr(lin, "qweight", None) is not None or not lin.gemv_ok(1)
-                            or not lin.weight.is_contiguous()):
-                        ok = False
-                        break
-                if not ok:
-                    break
-        if not ok:
-            return False
-        from ..ops import native as nat
-        cfg = self.cfg
-        return nat.decode_layers_supported(T, cfg.hidden_size, cfg.num_attention_heads, cfg.num_key_value_heads,
-                                           cfg.intermediate_size)
-
-    def _mega_table(self, cache) -> torch.Tensor:
-        """Per-layer pointer table of the whole-step kernel for this cache. Entries are tied to the cache object by a
-        weak reference, so a new cache that happens to reuse the id of a freed one gets a fresh table."""
-        import weakref
-        ent = self._mega_tables.get(id(cache))
-        sig = (self.layers[0].self_attn.qkv_proj.weight.data_ptr(), self.layers[-1].mlp.down_proj.weight.data_ptr(),
-               cache.k[0].data_ptr())
-        if ent is not None and ent[0]() is cache and ent[2] == sig:      # same cache object, weights not re-allocated
-            return ent[1]
-        for key in [k for k, e in self._mega_tables.items() if e[0]() is None]:
-            del self._mega_tables[key]
-        rows = []
+        if (cfg.attn_logit_softcap > 0 or getattr(self, "tp_world", 1) > 1 or cache.quant not in (None, "int8") or cache.window > 0
+                or cfg.hidden_size % 8 or cfg.intermediate_size % 8 or (cache.quant is None and cache.k[0].dtype != torch.bfloat16)):
+            return None
+        rows: List[int] = []
+        dt = torch.bfloat16
         for li, layer in enumerate(self.layers):
-            at, mlp = layer.self_attn, layer.mlp
-            rows.append([layer.input_layernorm.data_ptr(), at.qkv_proj.weight.data_ptr(),
-                         at.q_norm.data_ptr() if at.q_norm is not None else 0,
-                         at.k_norm.data_ptr() if at.k_norm is not None else 0, at.o_proj.weight.data_ptr(),
-                         layer.post_attention_layernorm.data_ptr(), mlp.gate_up_proj.weight.data_ptr(),
-                         mlp.down_proj.weight.data_ptr(), cache.k[li].data_ptr(), cache.v[li].data_ptr()])
-        t = torch.tensor(rows, dtype=torch.int64, device=self.embed_tokens.device)
-        self._mega_tables[id(cache)] = (weakref.ref(cache), t, sig)
-        return t
+            mods = layer._modules
+            at, mlp = mods["self_attn"], mods["mlp"]
+            if at.window or not isinstance(mlp, MLP):
+                return None
+            w = []
+            for lin in (at._modules["qkv_proj"], at._modules["o_proj"], mlp._modules["gate_up_proj"], mlp._modules["down_proj"]):
+                p, own = lin._parameters["weight"], lin.__dict__
+                if (lin._parameters.get("bias") is not None or lin._parameters.get("lora_a") is not None or own.get("lora_a") is not None
+                        or own.get("qweight") is not None or own.get("batched") is not None or p.requires_grad or p.dtype != dt
+                        or p.dim() != 2 or not p.is_contiguous() or p.data_ptr() % 16):
+                    return None
+                w.append(p.data_ptr())
+            norms = layer._parameters["input_layernorm"], layer._parameters["post_attention_layernorm"]
+            qk = (at._parameters["q_norm"], at._parameters["k_norm"]) if at.q_norm is not None else ()
+            if any(p.dtype != dt or p.data_ptr() % 16 for p in norms + qk):
+                return None
+            qn, kn = (p.data_ptr() for p in qk) if qk else (0, 0)
+            rows += [norms[0].data_ptr(), w[0], qn, kn, w[1], norms[1].data_ptr(), w[2], w[3], cache.k[li].data_ptr(),
+                     cache.v[li].data_ptr(), cache.k_scale[li].data_ptr() if cache.quant else 0,
+                     cache.v_scale[li].data_ptr() if cache.quant else 0]
+        return rows
 
     def _paged_attention_reference(self, qkv, at, rope, cache, meta, li, hq=None, hkv=None):
         from ..ops import reference as ref

@@ -215,6 +215,7 @@ def _bind_layer_split():
     LayerSplitDraft.forward_paged = DecoderLM.forward_paged
     LayerSplitDraft._paged_attention_reference = DecoderLM._paged_attention_reference
     LayerSplitDraft.rope = DecoderLM.rope
+    LayerSplitDraft._stack_addresses = DecoderLM._stack_addresses
 
 
 _bind_layer_split()

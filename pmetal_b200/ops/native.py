@@ -875,6 +875,37 @@ def _paged_on_tensor_cores(n_seq: int, max_q: int, max_kv: int, hq: int, hkv: in
     return new < 2.7 * n_seq * hkv * -(-max_q * rep // 64) * -(-max_kv // 64) / (2 * sms)
 
 
+def _paged_splits(n_seq: int, max_kv: int, hkv: int, max_q: int) -> int:
+    """Slices of the keys of a sequence, so that few sequences still occupy the machine. Steps of few tokens go by the bucket of
+    blocks that a captured decode step is built for, so that drafting and verifying cut the same keys alike and round alike."""
+    ctas, n_blocks = n_seq * hkv, -(-max_kv // 64)
+    if max_q <= 16:
+        n_blocks = max(8, 1 << (n_blocks - 1).bit_length())
+    return max(1, min(n_blocks // 4, 2 * sm_count() // max(ctas, 1), 32)) if ctas < sm_count() else 1
+
+
+def layer_stack(rows, x, meta, cos, sin, hq: int, hkv: int, inter: int, num_blocks: int, eps: float, scale: float):
+    """All layers of a dense decoder on the new tokens ``x`` [T, H] of a step, one call (csrc/layer_stack.cu). ``rows``: 12 device
+    addresses per layer, as pm_layer_stack takes them. Returns the last layer's output [T, H]."""
+    T, H = x.shape
+    n_seq = meta.block_table.shape[0]
+    n_layers = len(rows) // 12
+    tc = rows[10] == 0 and _paged_on_tensor_cores(n_seq, meta.max_q, meta.max_kv, hq, hkv)
+    n_split = 1 if tc else _paged_splits(n_seq, meta.max_kv, hkv, meta.max_q)
+    lib().pm_layer_stack_scratch.restype = c_ll
+    nbytes = lib().pm_layer_stack_scratch(c_int(T), c_int(H), c_int(hq), c_int(hkv), c_int(inter), c_int(n_split))
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    out = torch.empty_like(x)
+    global LAUNCHES
+    LAUNCHES += n_layers * (8 if T <= 128 else 9) - 1
+    _chk(lib().pm_layer_stack((c_ll * len(rows))(*rows), c_int(n_layers), _p(x), _p(out), _p(scratch), c_ll(nbytes), c_int(T), c_int(H),
+                              c_int(hq), c_int(hkv), c_int(inter), c_float(eps), c_float(scale), _p(cos), _p(sin), _p(meta.slots),
+                              _p(meta.block_table), _p(meta.seq_lens), _p(meta.q_start), _p(meta.q_lens), c_int(n_seq),
+                              c_int(meta.block_table.shape[1]), c_int(num_blocks), c_int(meta.max_q), c_int(int(tc)), c_int(n_split),
+                              _p(status_word(x.device)), _stream()), "pm_layer_stack")
+    return out
+
+
 def paged_attn(q, k_cache, v_cache, meta, scale: float, window: int = 0, n_split: int = 0, sink: int = 0,
                k_scale=None, v_scale=None, lut=None):
     """q: [total_q, hq, 128]; ``meta`` is a ``BatchMeta``. Long single sequences are split over key blocks.
@@ -892,9 +923,7 @@ def paged_attn(q, k_cache, v_cache, meta, scale: float, window: int = 0, n_split
                                     c_float(scale), _p(status_word(q.device)), _stream()), "pm_paged_attn_tc")
         return out
     if n_split <= 0:
-        ctas = n_seq * hkv
-        n_blocks = -(-meta.max_kv // 64)
-        n_split = max(1, min(n_blocks // 4, 2 * sm_count() // max(ctas, 1), 32)) if ctas < sm_count() else 1
+        n_split = _paged_splits(n_seq, meta.max_kv, hkv, meta.max_q)
     out = torch.empty_like(q)
     po = pml = None
     if n_split > 1:
@@ -1260,42 +1289,6 @@ def gdn_scan(q, k, v, g, beta, state=None):
 
 def gdn_scan_supported(dk: int, dv: int) -> bool:
     return dk in (64, 128) and dv in (64, 128)
-
-
-# ------------------------------------------------------------------------------------------- whole-step decode kernel
-def decode_layers_supported(M: int, H: int, hq: int, hkv: int, I: int) -> bool:
-    return bool(lib().pm_decode_layers_supported(c_int(M), c_int(H), c_int(hq), c_int(hkv), c_int(I)))
-
-
-def decode_layers(table, n_layers: int, x, scratch: dict, cos, sin, meta, hq: int, hkv: int, I: int, eps: float,
-                  scale: float):
-    """All decoder layers of one decode step in a single cooperative launch (csrc/decode_mega.cu). ``table`` is the
-    int64 device tensor of per-layer pointers, ``x`` [M, H] bf16 is updated in place, ``scratch`` holds the work
-    buffers made by ``decode_scratch``."""
-    M, H = x.shape
-    scratch["bar"].zero_()
-    _chk(lib().pm_decode_layers(_p(table), c_int(n_layers), c_int(M), c_int(H), c_int(hq), c_int(hkv), c_int(I),
-                                c_float(eps), c_float(scale), _p(x), _p(scratch["h"]), _p(scratch["qkv"]),
-                                _p(scratch["attn"]), _p(scratch["act"]), _p(scratch["part_o"]), _p(scratch["part_ml"]),
-                                _p(scratch["counters"]), _p(cos), _p(sin), _p(meta.block_table), _p(meta.seq_lens),
-                                _p(meta.slots), c_int(meta.block_table.shape[1]), c_int(scratch["n_split"]),
-                                _p(scratch["bar"]), _p(status_word(x.device)), _p(scratch.get("trace")), _stream()),
-         "pm_decode_layers")
-    return x
-
-
-def decode_splits(M: int, hkv: int, max_kv: int) -> int:
-    """CTAs per (row, kv head) in the attention phase: fill the grid, at least 64 keys per CTA, at most 16."""
-    return max(1, min(sm_count() // max(M * hkv, 1), 16, max(max_kv // 64, 1)))
-
-
-def decode_scratch(M: int, H: int, hq: int, hkv: int, I: int, n_split: int, device) -> dict:
-    bf = dict(dtype=torch.bfloat16, device=device)
-    return dict(h=torch.empty(M, H, **bf), qkv=torch.empty(M, (hq + 2 * hkv) * 128, **bf), attn=torch.empty(M, hq * 128, **bf),
-                act=torch.empty(M, I, **bf), part_o=torch.empty(n_split, M, hq, 128, dtype=torch.float32, device=device),
-                part_ml=torch.empty(n_split, M, hq, 2, dtype=torch.float32, device=device),
-                counters=torch.zeros(M * hkv, dtype=torch.int32, device=device),
-                bar=torch.zeros(2, dtype=torch.int32, device=device), n_split=n_split)
 
 
 # ------------------------------------------------------------------------------------------- fp32-stream decoders

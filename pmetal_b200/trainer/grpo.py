@@ -125,8 +125,8 @@ class GrpoStepStats:
 class RolloutWeights:
     """Context manager for the generation phase: every adapted projection is replaced by one bf16 weight
     W + s B A (refreshed from the current factors on entry, in buffers that keep their address from step to step), and
-    the factors are hidden, so that rollouts run on the adapter-free decode path (the whole-step kernel, the tensor-core
-    mat-vec and the CUDA graphs captured over them) instead of the slower adapter-aware one. The training forward is
+    the factors are hidden, so that rollouts run on the adapter-free decode path (one runtime call per step, the tensor-core
+    kernels for few rows and the CUDA graphs captured over them) instead of the slower adapter-aware one. The training forward is
     untouched: on exit the base weights and the factors are back. Packed (quantised) bases are left alone."""
 
     def __init__(self, model):
