@@ -53,11 +53,11 @@ extern "C" long long pm_layer_stack_scratch(int T, int H, int hq, int hkv, int I
 
 // layers: n_layers rows of 12 pointers on the host: input norm, q|k|v weight, q norm, k norm (0: none), output weight, post norm,
 // gate|up weight, down weight, key cache, value cache, key scales, value scales (0: bf16 cache, else int8). x: [T, H]; out: [T, H].
-// tensor_cores 1: attention through pm_paged_attn_tc, else pm_paged_attn_ex with n_split. Returns the first launcher's error.
+// route: attention through 0 pm_paged_attn_ex with n_split, 1 pm_paged_attn_tc, 2 pm_paged_decode. Returns the first launcher's error.
 extern "C" int pm_layer_stack(const long long* layers, int n_layers, const void* x, void* out, void* scratch, long long scratch_bytes,
                               int T, int H, int hq, int hkv, int I, float eps, float scale, const float* cs, const float* sn,
                               const long long* slots, const int* block_table, const int* seq_lens, const int* q_start,
-                              const int* q_lens, int num_seqs, int max_blocks, int num_blocks, int max_q, int tensor_cores, int n_split,
+                              const int* q_lens, int num_seqs, int max_blocks, int num_blocks, int max_q, int route, int n_split,
                               int* status, cudaStream_t st) {
   if (T <= 0 || n_layers <= 0 || H % 8 || I % 8 || hkv <= 0 || hq % hkv) return -1;
   if (scratch_bytes < pm_layer_stack_scratch(T, H, hq, hkv, I, n_split) || (reinterpret_cast<uintptr_t>(scratch) & 15)) return -2;
@@ -99,11 +99,13 @@ extern "C" int pm_layer_stack(const long long* layers, int n_layers, const void*
     } else if ((rc = pm_qknorm_rope_cache(qkv, ld, ptr(2), ptr(3), cs, sn, q, ptr(8), ptr(9), slots, T, hq, hkv, eps, st))) {
       return rc;
     }
-    rc = tensor_cores ? pm_paged_attn_tc(q, ptr(8), ptr(9), o, block_table, seq_lens, q_start, q_lens, num_seqs, max_blocks, num_blocks, T,
+    float *ksc = static_cast<float*>(ptr(10)), *vsc = static_cast<float*>(ptr(11));
+    rc = route == 2 ? pm_paged_decode(q, ptr(8), ptr(9), ksc, vsc, o, block_table, seq_lens, q_start, q_lens, num_seqs, max_blocks, num_blocks,
+                                      max_q, hq, hkv, scale, 0, status, st)
+         : route == 1 ? pm_paged_attn_tc(q, ptr(8), ptr(9), o, block_table, seq_lens, q_start, q_lens, num_seqs, max_blocks, num_blocks, T,
                                          max_q, hq, hkv, scale, status, st)
                       : pm_paged_attn_ex(q, ptr(8), ptr(9), o, block_table, seq_lens, q_start, q_lens, part_o, part_ml, num_seqs,
-                                         max_blocks, T, max_q, hq, hkv, n_split, scale, 0, 0, static_cast<float*>(ptr(10)),
-                                         static_cast<float*>(ptr(11)), st);
+                                         max_blocks, T, max_q, hq, hkv, n_split, scale, 0, 0, ksc, vsc, st);
     if (rc) return rc;
     if ((rc = s.linear(o, hq * 128, ptr(4), H, h, x))) return rc;
     if ((rc = pm_rmsnorm_fwd(h, nullptr, ptr(5), y, nullptr, rstd, T, H, eps, st))) return rc;

@@ -286,12 +286,11 @@ int pm_latent_take(const void* o128, int n, int H, int dv, void* out, long long 
 long long pm_layer_stack_scratch(int T, int H, int hq, int hkv, int I, int n_split);
 // layers: n_layers rows of 12 pointers on the host: input norm, q|k|v weight, q norm, k norm (0: none), output weight, post norm,
 // gate|up weight, down weight, key cache, value cache, key scales, value scales (0: bf16 cache, else int8). x: [T, H]; out: [T, H].
-// tensor_cores 1: attention through pm_paged_attn_tc, else pm_paged_attn_ex with n_split. Returns the first launcher's error.
+// route: attention through 0 pm_paged_attn_ex with n_split, 1 pm_paged_attn_tc, 2 pm_paged_decode. Returns the first launcher's error.
 int pm_layer_stack(const long long* layers, int n_layers, const void* x, void* out, void* scratch, long long
     scratch_bytes, int T, int H, int hq, int hkv, int I, float eps, float scale, const float* cs, const float* sn,
     const long long* slots, const int* block_table, const int* seq_lens, const int* q_start, const int* q_lens, int
-    num_seqs, int max_blocks, int num_blocks, int max_q, int tensor_cores, int n_split, int* status, cudaStream_t
-    st);
+    num_seqs, int max_blocks, int num_blocks, int max_q, int route, int n_split, int* status, cudaStream_t st);
 
 // ---------------------------------------------------------------- linear_attn.cu
 // Token-by-token recurrence. u [tokens, ldu]; cs / sn fp32 [tokens, R / 2] (unused when R is 0); rot: 1 pairs (i, i + R / 2),
@@ -396,6 +395,14 @@ int pm_moe_combine(const void* z, const int* inv, const float* w, int k, void* y
 int pm_gguf_dequant_bf16(const void* src, void* dst, long long n, int type, cudaStream_t st);
 int pm_fp8_quant(const void* x, void* q, float* scales, long long n, cudaStream_t st);
 int pm_fp8_dequant(const void* q, const float* scales, void* y, long long n, cudaStream_t st);
+
+// ---------------------------------------------------------------- paged_decode.cu
+// q, out: [total_q, hq, 128]; caches, table and lengths as for pm_paged_attn_ex, no window. k_scale / v_scale null: bf16 cache. Token i of
+// sequence s sees the keys j <= seq_lens[s] - q_lens[s] + i. hq / hkv up to 8. splits 0: chosen here (1, 2, 4 or 8 slices of the keys).
+int pm_paged_decode(const void* q, const void* k_cache, const void* v_cache, const float* k_scale, const float*
+    v_scale, void* out, const int* block_table, const int* seq_lens, const int* q_start, const int* q_lens, int
+    num_seqs, int max_blocks, int num_blocks, int max_q, int hq, int hkv, float scale, int splits, int* status,
+    cudaStream_t st);
 
 // ---------------------------------------------------------------- postnorm.cu
 // xf [n, width] fp32 = table[ids] * scale, xc the same in the table's type (nullable). f32: the table is fp32, else bf16.

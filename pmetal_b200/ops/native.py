@@ -875,13 +875,25 @@ def _paged_on_tensor_cores(n_seq: int, max_q: int, max_kv: int, hq: int, hkv: in
     return new < 2.7 * n_seq * hkv * -(-max_q * rep // 64) * -(-max_kv // 64) / (2 * sms)
 
 
-def _paged_splits(n_seq: int, max_kv: int, hkv: int, max_q: int) -> int:
-    """Slices of the keys of a sequence, so that few sequences still occupy the machine. Steps of few tokens go by the bucket of
-    blocks that a captured decode step is built for, so that drafting and verifying cut the same keys alike and round alike."""
+PAGED_SPLIT, PAGED_TENSOR, PAGED_DECODE = 0, 1, 2
+
+
+def _paged_splits(n_seq: int, max_kv: int, hkv: int) -> int:
+    """Slices of the keys of a sequence for the 64-row kernel, so that few sequences still occupy the machine."""
     ctas, n_blocks = n_seq * hkv, -(-max_kv // 64)
-    if max_q <= 16:
-        n_blocks = max(8, 1 << (n_blocks - 1).bit_length())
     return max(1, min(n_blocks // 4, 2 * sm_count() // max(ctas, 1), 32)) if ctas < sm_count() else 1
+
+
+def _paged_route(meta, hq: int, hkv: int, int8: bool):
+    """(kernel, slices of the keys) for attention over a bf16 or int8 paged cache without a window: steps of up to 8 tokens per sequence
+    and 8 heads per group stream the keys once per token (csrc/paged_decode.cu), prompts fill tensor-core tiles where
+    ``_paged_on_tensor_cores`` says so, the rest goes to the 64-row kernel."""
+    n_seq = meta.block_table.shape[0]
+    if meta.max_q <= 8 and hq // hkv <= 8:
+        return PAGED_DECODE, 1
+    if not int8 and _paged_on_tensor_cores(n_seq, meta.max_q, meta.max_kv, hq, hkv):
+        return PAGED_TENSOR, 1
+    return PAGED_SPLIT, _paged_splits(n_seq, meta.max_kv, hkv)
 
 
 def layer_stack(rows, x, meta, cos, sin, hq: int, hkv: int, inter: int, num_blocks: int, eps: float, scale: float):
@@ -890,8 +902,7 @@ def layer_stack(rows, x, meta, cos, sin, hq: int, hkv: int, inter: int, num_bloc
     T, H = x.shape
     n_seq = meta.block_table.shape[0]
     n_layers = len(rows) // 12
-    tc = rows[10] == 0 and _paged_on_tensor_cores(n_seq, meta.max_q, meta.max_kv, hq, hkv)
-    n_split = 1 if tc else _paged_splits(n_seq, meta.max_kv, hkv, meta.max_q)
+    route, n_split = _paged_route(meta, hq, hkv, rows[10] != 0)
     lib().pm_layer_stack_scratch.restype = c_ll
     nbytes = lib().pm_layer_stack_scratch(c_int(T), c_int(H), c_int(hq), c_int(hkv), c_int(inter), c_int(n_split))
     scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
@@ -901,7 +912,7 @@ def layer_stack(rows, x, meta, cos, sin, hq: int, hkv: int, inter: int, num_bloc
     _chk(lib().pm_layer_stack((c_ll * len(rows))(*rows), c_int(n_layers), _p(x), _p(out), _p(scratch), c_ll(nbytes), c_int(T), c_int(H),
                               c_int(hq), c_int(hkv), c_int(inter), c_float(eps), c_float(scale), _p(cos), _p(sin), _p(meta.slots),
                               _p(meta.block_table), _p(meta.seq_lens), _p(meta.q_start), _p(meta.q_lens), c_int(n_seq),
-                              c_int(meta.block_table.shape[1]), c_int(num_blocks), c_int(meta.max_q), c_int(int(tc)), c_int(n_split),
+                              c_int(meta.block_table.shape[1]), c_int(num_blocks), c_int(meta.max_q), c_int(route), c_int(n_split),
                               _p(status_word(x.device)), _stream()), "pm_layer_stack")
     return out
 
@@ -914,16 +925,24 @@ def paged_attn(q, k_cache, v_cache, meta, scale: float, window: int = 0, n_split
     total_q, hq, _ = q.shape
     hkv = k_cache.shape[2]
     n_seq = meta.block_table.shape[0]
-    if (n_split <= 0 and k_scale is None and window <= 0 and _paged_on_tensor_cores(n_seq, meta.max_q, meta.max_kv, hq, hkv)
-            and q.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous()):
-        out = torch.empty_like(q)
-        _chk(lib().pm_paged_attn_tc(_p(q), _p(k_cache), _p(v_cache), _p(out), _p(meta.block_table), _p(meta.seq_lens),
-                                    _p(meta.q_start), _p(meta.q_lens), c_int(n_seq), c_int(meta.block_table.shape[1]),
-                                    c_int(k_cache.shape[0]), c_int(total_q), c_int(meta.max_q), c_int(hq), c_int(hkv),
-                                    c_float(scale), _p(status_word(q.device)), _stream()), "pm_paged_attn_tc")
-        return out
+    if n_split <= 0 and window <= 0 and lut is None and q.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous():
+        route, _ = _paged_route(meta, hq, hkv, k_scale is not None)
+        if route == PAGED_DECODE:
+            out = torch.empty_like(q)
+            _chk(lib().pm_paged_decode(_p(q), _p(k_cache), _p(v_cache), _p(k_scale), _p(v_scale), _p(out), _p(meta.block_table),
+                                       _p(meta.seq_lens), _p(meta.q_start), _p(meta.q_lens), c_int(n_seq),
+                                       c_int(meta.block_table.shape[1]), c_int(k_cache.shape[0]), c_int(meta.max_q), c_int(hq), c_int(hkv),
+                                       c_float(scale), c_int(0), _p(status_word(q.device)), _stream()), "pm_paged_decode")
+            return out
+        if route == PAGED_TENSOR:
+            out = torch.empty_like(q)
+            _chk(lib().pm_paged_attn_tc(_p(q), _p(k_cache), _p(v_cache), _p(out), _p(meta.block_table), _p(meta.seq_lens),
+                                        _p(meta.q_start), _p(meta.q_lens), c_int(n_seq), c_int(meta.block_table.shape[1]),
+                                        c_int(k_cache.shape[0]), c_int(total_q), c_int(meta.max_q), c_int(hq), c_int(hkv),
+                                        c_float(scale), _p(status_word(q.device)), _stream()), "pm_paged_attn_tc")
+            return out
     if n_split <= 0:
-        n_split = _paged_splits(n_seq, meta.max_kv, hkv, meta.max_q)
+        n_split = _paged_splits(n_seq, meta.max_kv, hkv)
     out = torch.empty_like(q)
     po = pml = None
     if n_split > 1:

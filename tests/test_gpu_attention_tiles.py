@@ -6,7 +6,7 @@ pytestmark = pytest.mark.gpu
 
 
 def _rel(a, b):
-    return float((a.float() - b.float()).norm() / b.float().norm())
+    return float((a.detach().float() - b.detach().float()).norm() / b.detach().float().norm())
 
 
 def _dense(q, k, v, first, limit, scale):
@@ -54,6 +54,47 @@ def test_paged_prompt_attention(hq, hkv, lens, qlens):
         assert _rel(out[at:at + m], want) < 6e-3, (i, n, m)
         at += m
     nat.check_status()
+
+
+# (kv lengths, new tokens): ends on and beside the 16-key quarters and the 64-key blocks, fewer blocks than slices, several tokens
+DECODE = [([1, 15, 16, 17], [1, 1, 1, 1]), ([63, 64, 65, 700], [1, 1, 1, 1]), ([130, 5], [5, 2]), ([2100], [8])]
+
+
+@pytest.mark.parametrize("quant", [None, "int8"])
+@pytest.mark.parametrize("hq,hkv", [(2, 2), (4, 2), (8, 1), (6, 2)])
+@pytest.mark.parametrize("lens,qlens", DECODE)
+@pytest.mark.parametrize("splits", [0, 1, 2, 8])
+def test_paged_decode_attention(quant, hq, hkv, lens, qlens, splits):
+    from pmetal_b200.models.kv_cache import PagedKVCache
+    from pmetal_b200.ops import native as nat
+    g = torch.Generator(device="cuda").manual_seed(sum(lens) + hq)
+    cache = PagedKVCache(1, hkv, 128, 64, quant=quant)
+    cache.free = torch.randperm(64, generator=torch.Generator().manual_seed(3)).tolist()
+    for i, (n, m) in enumerate(zip(lens, qlens)):
+        cache.add_sequence(i)
+        if n > m:
+            cache.reserve(i, n - m)
+    meta = cache.prepare(list(range(len(lens))), qlens)
+    every = torch.arange(64 * 64, device="cuda")
+    k, v = (torch.randn(64 * 64, hkv, 128, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    cache.write_reference(0, k, v * 0.01, every)         # small values: the scales of the int8 cache matter
+    q = torch.randn(sum(qlens), hq, 128, device="cuda", generator=g).to(torch.bfloat16)
+    out = torch.full_like(q, float("nan"))
+    p = nat._p
+    scales = (cache.k_scale[0], cache.v_scale[0]) if quant else (None, None)
+    rc = nat.lib().pm_paged_decode(p(q), p(cache.k[0]), p(cache.v[0]), p(scales[0]), p(scales[1]), p(out), p(meta.block_table),
+                                   p(meta.seq_lens), p(meta.q_start), p(meta.q_lens), nat.c_int(len(lens)),
+                                   nat.c_int(meta.block_table.shape[1]), nat.c_int(64), nat.c_int(max(qlens)), nat.c_int(hq),
+                                   nat.c_int(hkv), nat.c_float(128 ** -0.5), nat.c_int(splits), p(nat.status_word(q.device)), nat._stream())
+    assert rc == 0
+    cache.compute_dtype = torch.float32                  # the oracle reads codes times scales unrounded
+    at = 0
+    for i, (n, m) in enumerate(zip(lens, qlens)):
+        kk, vv = cache.gather(0, i)
+        lim = torch.arange(n - m, n, device="cuda")
+        want = _dense(q[at:at + m], kk, vv, torch.zeros_like(lim), lim, 128 ** -0.5)
+        assert _rel(out[at:at + m], want) < 5e-3, (i, n, m)      # bf16 probabilities and outputs: 2^-9 each
+        at += m
 
 
 def test_paged_dispatch_keeps_small_steps_on_the_split_kernel():
