@@ -28,6 +28,15 @@ struct SkinnyParams {
   int nkb, per, splits, stages, swiglu;
   float alpha;
   int* status;
+  // RMSNorm around the product (nullable). In: x holds rows times the norm's weight, ss_in [parts_in][128] partial sums of squares of
+  // the rows themselves, so that a row's 1 / rms is a factor of its sums. Out: the same pair for the next norm, y2 = y * nw_out and
+  // the sum of squares of every column tile, ss_out [tiles][128].
+  const float* ss_in;
+  int parts_in;
+  float eps;
+  const __nv_bfloat16* nw_out;
+  __nv_bfloat16* y2;
+  float* ss_out;
 };
 
 constexpr int kSkW = 128 * 64 * 2;        // one k block of a weight tile: 16 KB
@@ -46,7 +55,7 @@ __device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
 // Sum over the cluster and epilogue of this CTA's share of the token rows, one warp per row; all loads of a row are in flight
 // together. Ends with this thread's arrival at the cluster barrier behind which the partial tiles may go away.
 template <int kSplits>
-__device__ __forceinline__ void skinny_finish(const SkinnyParams& p, uint32_t part, int split, int n0) {
+__device__ __forceinline__ void skinny_finish(const SkinnyParams& p, uint32_t part, int split, int n0, const float* s_rstd) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t at[kSplits];
 #pragma unroll
@@ -54,6 +63,7 @@ __device__ __forceinline__ void skinny_finish(const SkinnyParams& p, uint32_t pa
   const int n = n0 + lane * (p.swiglu ? 2 : 4);
   for (int m = split + kSplits * warp; m < p.M; m += kSplits * (kThreads / 32)) {
     float f[4] = {0.f, 0.f, 0.f, 0.f};
+    const float alpha = p.ss_in ? p.alpha * s_rstd[m] : p.alpha;
     if (p.swiglu) {
       float2 g[kSplits], u[kSplits];
 #pragma unroll
@@ -66,7 +76,7 @@ __device__ __forceinline__ void skinny_finish(const SkinnyParams& p, uint32_t pa
       if (n < p.N) {                  // N is even
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const float gv = f[e] * p.alpha, uv = f[2 + e] * p.alpha;
+          const float gv = f[e] * alpha, uv = f[2 + e] * alpha;
           f[e] = gv / (1.f + __expf(-gv)) * uv;
         }
         if (p.res) {
@@ -84,10 +94,26 @@ __device__ __forceinline__ void skinny_finish(const SkinnyParams& p, uint32_t pa
       if (p.res && n < p.N) rv = *reinterpret_cast<const uint2*>(p.res + m * p.ldr + n);
 #pragma unroll
       for (int c = 0; c < kSplits; ++c) { f[0] += v[c].x; f[1] += v[c].y; f[2] += v[c].z; f[3] += v[c].w; }
+      float ss = 0.f;
       if (n < p.N) {                  // N is a multiple of 8
-        f[0] = fmaf(f[0], p.alpha, bf16_bits_to_float(rv.x & 0xFFFFu)); f[1] = fmaf(f[1], p.alpha, bf16_bits_to_float(rv.x >> 16));
-        f[2] = fmaf(f[2], p.alpha, bf16_bits_to_float(rv.y & 0xFFFFu)); f[3] = fmaf(f[3], p.alpha, bf16_bits_to_float(rv.y >> 16));
-        *reinterpret_cast<uint2*>(p.y + m * p.ldy + n) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
+        f[0] = fmaf(f[0], alpha, bf16_bits_to_float(rv.x & 0xFFFFu)); f[1] = fmaf(f[1], alpha, bf16_bits_to_float(rv.x >> 16));
+        f[2] = fmaf(f[2], alpha, bf16_bits_to_float(rv.y & 0xFFFFu)); f[3] = fmaf(f[3], alpha, bf16_bits_to_float(rv.y >> 16));
+        const uint2 yv = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
+        *reinterpret_cast<uint2*>(p.y + m * p.ldy + n) = yv;
+        if (p.y2) {
+          const uint2 nv = *reinterpret_cast<const uint2*>(p.nw_out + n);
+          const float y[4] = {bf16_bits_to_float(yv.x & 0xFFFFu), bf16_bits_to_float(yv.x >> 16), bf16_bits_to_float(yv.y & 0xFFFFu),
+                              bf16_bits_to_float(yv.y >> 16)};
+          ss = y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3];
+          *reinterpret_cast<uint2*>(p.y2 + m * p.ldy + n) =
+              make_uint2(pack_bf16x2(y[0] * bf16_bits_to_float(nv.x & 0xFFFFu), y[1] * bf16_bits_to_float(nv.x >> 16)),
+                         pack_bf16x2(y[2] * bf16_bits_to_float(nv.y & 0xFFFFu), y[3] * bf16_bits_to_float(nv.y >> 16)));
+        }
+      }
+      if (p.y2) {
+#pragma unroll
+        for (int e = 16; e > 0; e >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, e);
+        if (lane == 0) p.ss_out[(n0 >> 7) * 128 + m] = ss;
       }
     }
   }
@@ -107,6 +133,7 @@ skinny_linear_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], done_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
+  __shared__ float s_rstd[128];
   volatile int* abort_flag = &abort_word;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -191,6 +218,13 @@ skinny_linear_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     // ------------------------------------------------------------------ accumulator -> shared memory, [token][weight row]
     float* part = reinterpret_cast<float*>(smem);
     const int r = (warp & 3) * 32 + lane;
+    if (p.ss_in) {                    // while the products are on their way
+      pdl_wait();
+      float ss = 0.f;
+      if (r < p.M)
+        for (int i = 0; i < p.parts_in; ++i) ss += __ldcg(p.ss_in + i * 128 + r);
+      s_rstd[r] = rsqrtf(ss / static_cast<float>(p.K) + p.eps);
+    }
     const bool have = nkb > 0 && mbar_wait(&done_bar, 0, abort_flag, p.status, kTimeoutEpilogue);
     tc_fence_after();
     const uint32_t t0 = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
@@ -213,16 +247,48 @@ skinny_linear_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   if (p.splits > 1) cluster_sync_all();
   if (warp != 0) pdl_wait();          // the residual and the output belong to earlier kernels until here (warp 0 has waited)
   switch (p.splits) {
-    case 1: skinny_finish<1>(p, smem_u32(smem), split, n0); break;
-    case 2: skinny_finish<2>(p, smem_u32(smem), split, n0); break;
-    case 4: skinny_finish<4>(p, smem_u32(smem), split, n0); break;
-    default: skinny_finish<8>(p, smem_u32(smem), split, n0); break;
+    case 1: skinny_finish<1>(p, smem_u32(smem), split, n0, s_rstd); break;
+    case 2: skinny_finish<2>(p, smem_u32(smem), split, n0, s_rstd); break;
+    case 4: skinny_finish<4>(p, smem_u32(smem), split, n0, s_rstd); break;
+    default: skinny_finish<8>(p, smem_u32(smem), split, n0, s_rstd); break;
   }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, kCols);
   }
   if (p.splits > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // the peers have read this CTA's partial tile
+}
+
+// What a chain that starts from plain rows needs: x * nw and the rows' sums of squares. One CTA per row.
+__global__ void __launch_bounds__(256) skinny_prep_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ nw,
+                                                          __nv_bfloat16* __restrict__ y2, float* __restrict__ ss_out, int H) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float red[8];
+  const long long base = static_cast<long long>(blockIdx.x) * H;
+  float ss = 0.f;
+  for (int c = threadIdx.x * 4; c < H; c += 1024) {
+    const uint2 xv = *reinterpret_cast<const uint2*>(x + base + c), nv = *reinterpret_cast<const uint2*>(nw + c);
+    const uint32_t xw[2] = {xv.x, xv.y}, nq[2] = {nv.x, nv.y};
+    uint32_t o[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float a = bf16_bits_to_float(xw[e] & 0xFFFFu), b = bf16_bits_to_float(xw[e] >> 16);
+      ss += a * a + b * b;
+      o[e] = pack_bf16x2(a * bf16_bits_to_float(nq[e] & 0xFFFFu), b * bf16_bits_to_float(nq[e] >> 16));
+    }
+    *reinterpret_cast<uint2*>(y2 + base + c) = make_uint2(o[0], o[1]);
+  }
+#pragma unroll
+  for (int e = 16; e > 0; e >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, e);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t += red[i];
+    ss_out[blockIdx.x] = t;
+  }
 }
 
 template <int kMT>
@@ -264,21 +330,25 @@ static int launch_skinny(const CUtensorMap& mw, const CUtensorMap& mx, SkinnyPar
 
 using namespace pm;
 
-// x: [M, K] rows ldx apart, w: [N, K] (swiglu: [2 N, K], gate rows first) rows ldw apart, y / res: [M, N] rows ldy / ldr apart (res
-// nullable, may be y). M <= 128; K, N and the row strides multiples of 8, pointers 16-byte aligned. splits 0: chosen here. chain: see
-// the head of this file. Returns a negative value for arguments outside of that.
-extern "C" int pm_linear_skinny(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy, const void* res,
-                                long long ldr, int M, int N, int K, int swiglu, float alpha, int splits, int chain, int* status,
-                                cudaStream_t st) {
+// pm_linear_skinny inside a chain of RMSNorms. ss_in non-null: x is rows * norm weight and ss_in [parts_in][128] their partial sums of squares
+// (row m of part i at i * 128 + m), the product is that of the normalised rows. y2 non-null (not with swiglu): y2 = y * nw_out with y's
+// strides and ss_out [(N + 127) / 128][128] for the next link.
+extern "C" int pm_linear_skinny_norm(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy, const void* res,
+                                     long long ldr, int M, int N, int K, int swiglu, float alpha, int splits, int chain,
+                                     const float* ss_in, int parts_in, float eps, const void* nw_out, void* y2, float* ss_out,
+                                     int* status, cudaStream_t st) {
   if (M <= 0 || M > 128 || N <= 0 || K <= 0) return -1;
   if ((N | K) % 8 || (ldx | ldw | ldy) % 8 || (res && ldr % 8)) return -2;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) |
-       reinterpret_cast<uintptr_t>(res)) & 15)
+       reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(y2) | reinterpret_cast<uintptr_t>(nw_out)) & 15)
     return -3;
+  if (y2 && (swiglu || !nw_out || !ss_out)) return -5;
   SkinnyParams p{};
   p.y = static_cast<__nv_bfloat16*>(y); p.ldy = ldy;
   p.res = static_cast<const __nv_bfloat16*>(res); p.ldr = ldr;
   p.M = M; p.N = N; p.K = K; p.swiglu = swiglu; p.alpha = alpha; p.status = status;
+  p.ss_in = ss_in; p.parts_in = parts_in; p.eps = eps;
+  p.nw_out = static_cast<const __nv_bfloat16*>(nw_out); p.y2 = static_cast<__nv_bfloat16*>(y2); p.ss_out = ss_out;
   p.nkb = (K + kBK - 1) / kBK;
   const int rows = swiglu ? 64 : 128, tiles = (N + rows - 1) / rows;
   if (splits <= 0) {
@@ -300,4 +370,22 @@ extern "C" int pm_linear_skinny(const void* x, long long ldx, const void* w, lon
     case 64: return launch_skinny<64>(mw, mx, p, tiles, chain, st);
     default: return launch_skinny<128>(mw, mx, p, tiles, chain, st);
   }
+}
+
+// x: [M, K] rows ldx apart, w: [N, K] (swiglu: [2 N, K], gate rows first) rows ldw apart, y / res: [M, N] rows ldy / ldr apart (res
+// nullable, may be y). M <= 128; K, N and the row strides multiples of 8, pointers 16-byte aligned. splits 0: chosen here. chain: see
+// the head of this file. Returns a negative value for arguments outside of that.
+extern "C" int pm_linear_skinny(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy, const void* res,
+                                long long ldr, int M, int N, int K, int swiglu, float alpha, int splits, int chain, int* status,
+                                cudaStream_t st) {
+  return pm_linear_skinny_norm(x, ldx, w, ldw, y, ldy, res, ldr, M, N, K, swiglu, alpha, splits, chain, nullptr, 0, 0.f, nullptr, nullptr,
+                               nullptr, status, st);
+}
+
+// First link of such a chain: y2 = x * nw [M, H] and ss [128] = the rows' sums of squares. M <= 128, H a multiple of 8.
+extern "C" int pm_skinny_prep(const void* x, const void* nw, void* y2, float* ss, int M, int H, cudaStream_t st) {
+  if (M <= 0 || M > 128 || H <= 0 || H % 8) return -1;
+  return static_cast<int>(launch_pdl(skinny_prep_kernel, dim3(static_cast<unsigned>(M)), dim3(256), 0, st,
+                                     static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(nw),
+                                     static_cast<__nv_bfloat16*>(y2), ss, H));
 }

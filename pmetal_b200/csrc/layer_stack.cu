@@ -1,12 +1,15 @@
 // The cached forward of all layers of a dense decoder in one call: the host side of a prompt or of a decode step.
 //
-// A layer is eight launches (norm, q|k|v, head norm + rope + cache append, attention, output projection, norm, gate|up, down).
+// A layer is eight or nine launches (norm, q|k|v, head norm + rope + cache append, attention, output projection, norm, gate|up, its
+// unit, down).
 // Issued one by one through the interpreter they cost about 35 us of host time each, 12 ms for 28 layers, whatever the
 // number of tokens; issued here a launch costs 2 to 4 us. Nothing is allocated and nothing is kept between calls: the
 // caller passes the layer pointers, a scratch buffer and the step's metadata.
 //
-// Up to 128 tokens the linear layers run on gemm_skinny.cu and every kernel of the chain is launched with programmatic
-// stream serialization (pdl.cuh); above that on the tile GEMMs.
+// Up to 128 tokens the linear layers run on gemm_skinny.cu, and the norms are part of them: the projection that writes the residual
+// stream also writes it times the next norm's weight, with the rows' sums of squares, and the next projection multiplies its sums
+// by 1 / rms. That leaves six kernels, each launched with programmatic stream serialization (pdl.cuh). A decode step of 28
+// layers: one row 898 us with norm kernels, 838 us without; 64 rows 1803, 1791 us. Above 128 tokens the tile GEMMs run.
 #include <stdint.h>
 
 #include <algorithm>
@@ -22,16 +25,27 @@ constexpr int kSkinnyRows = 128;
 
 struct Stack {
   int T;
+  float eps;
   int* status;
   cudaStream_t st;
-  int linear(const void* x, int K, const void* w, int N, void* y, const void* res) const {
-    if (T <= kSkinnyRows) return pm_linear_skinny(x, K, w, K, y, N, res, N, T, N, K, 0, 1.f, 0, 1, status, st);
+  // more than kSkinnyRows tokens
+  int tile(const void* x, int K, const void* w, int N, void* y, const void* res) const {
     const int bn = N >= 256 ? 256 : N >= 128 ? 128 : N >= 64 ? 64 : 32;
     if (T >= 256 && bn >= 128)
       return pm_gemm_bf16_2sm(x, 0, K, T, w, 0, K, N, nullptr, 0, 0, 0, nullptr, 0, 0, 0, y, 0, N, res, res ? N : 0, T, N, K, 0, 0, 1.f, 1,
                               0, nullptr, 0, 0, nullptr, 0, 0, status, st);
     return pm_gemm_bf16(x, 0, K, T, w, 0, K, N, nullptr, 0, 0, 0, nullptr, 0, 0, 0, y, 0, N, res, res ? N : 0, T, N, K, 0, 0, 1.f, bn, 1, 0,
                         nullptr, 0, 0, nullptr, 0, nullptr, 0, nullptr, 0, 0, status, st);
+  }
+  // up to kSkinnyRows: reads the pair (rows * norm weight, sums of squares in `parts` parts)
+  int normed(const void* xw, const float* ss, int parts, int K, const void* w, int N, void* y, int swiglu) const {
+    return pm_linear_skinny_norm(xw, K, w, K, y, N, nullptr, 0, T, N, K, swiglu, 1.f, 0, 1, ss, parts, eps, nullptr, nullptr, nullptr, status,
+                                 st);
+  }
+  // writes the residual stream and, where a norm follows (nw), the next pair
+  int residual(const void* x, int K, const void* w, int N, void* y, const void* res, const void* nw, void* yw, float* ss) const {
+    return pm_linear_skinny_norm(x, K, w, K, y, N, res, N, T, N, K, 0, 1.f, 0, 1, nullptr, 0, 0.f, nw, nw ? yw : nullptr, nw ? ss : nullptr,
+                                 status, st);
   }
 };
 
@@ -45,7 +59,7 @@ extern "C" long long pm_layer_stack_scratch(int T, int H, int hq, int hkv, int I
   const long long d = 128, t = T;
   long long n = 0;
   auto add = [&](long long b) { n += (b + 255) / 256 * 256; };
-  add(2 * t * H); add(4 * t); add(2 * t * (hq + 2 * hkv) * d); add(2 * t * hq * d); add(2 * t * hkv * d); add(2 * t * hq * d);
+  add(2 * t * H); add(T <= kSkinnyRows ? 4ll * 128 * ((H + 127) / 128) : 4 * t); add(2 * t * (hq + 2 * hkv) * d); add(2 * t * hq * d); add(2 * t * hkv * d); add(2 * t * hq * d);
   add(2 * t * H); add(2 * t * H); add(T <= kSkinnyRows ? 0 : 4 * t * I); add(2 * t * I);
   if (n_split > 1) { add(4ll * n_split * t * hq * d); add(8ll * n_split * t * hq); }
   return n;
@@ -70,7 +84,9 @@ extern "C" int pm_layer_stack(const long long* layers, int n_layers, const void*
     return b;
   };
   void* y = buf(2ll * T * H);
-  float* rstd = static_cast<float*>(buf(4ll * T));
+  const bool few = T <= kSkinnyRows;
+  const int parts = (H + 127) / 128;
+  float* rstd = static_cast<float*>(buf(few ? 4ll * 128 * parts : 4ll * T));   // few tokens: the sums of squares
   char* qkv = static_cast<char*>(buf(2ll * T * ld));
   void* q = buf(2ll * T * hq * d);
   void* k = buf(2ll * T * hkv * d);
@@ -81,15 +97,20 @@ extern "C" int pm_layer_stack(const long long* layers, int n_layers, const void*
   void* act = buf(2ll * T * I);
   float* part_o = n_split > 1 ? static_cast<float*>(buf(4ll * n_split * T * hq * d)) : nullptr;
   float* part_ml = n_split > 1 ? static_cast<float*>(buf(8ll * n_split * T * hq)) : nullptr;
-  const Stack s{T, status, st};
-  const PdlScope scope(T <= kSkinnyRows);
+  const Stack s{T, eps, status, st};
+  const PdlScope scope(few);
   int rc;
+  if (few && (rc = pm_skinny_prep(x, reinterpret_cast<void*>(layers[0]), y, rstd, T, H, st))) return rc;
   for (int l = 0; l < n_layers; ++l) {
     const long long* p = layers + 12ll * l;
     auto ptr = [&](int i) { return reinterpret_cast<void*>(p[i]); };
     const bool q8 = p[10] != 0;
-    if ((rc = pm_rmsnorm_fwd(x, nullptr, ptr(0), y, nullptr, rstd, T, H, eps, st))) return rc;
-    if ((rc = s.linear(y, H, ptr(1), ld, qkv, nullptr))) return rc;
+    if (few) {
+      if ((rc = s.normed(y, rstd, l ? parts : 1, H, ptr(1), ld, qkv, 0))) return rc;
+    } else {
+      if ((rc = pm_rmsnorm_fwd(x, nullptr, ptr(0), y, nullptr, rstd, T, H, eps, st))) return rc;
+      if ((rc = s.tile(y, H, ptr(1), ld, qkv, nullptr))) return rc;
+    }
     if (q8) {
       void* v = qkv + (hq + hkv) * d * 2;
       if ((rc = pm_qknorm_rope_fwd(qkv, ld, ptr(2), ptr(3), cs, sn, q, k, T, hq, hkv, eps, st))) return rc;
@@ -107,16 +128,19 @@ extern "C" int pm_layer_stack(const long long* layers, int n_layers, const void*
                       : pm_paged_attn_ex(q, ptr(8), ptr(9), o, block_table, seq_lens, q_start, q_lens, part_o, part_ml, num_seqs,
                                          max_blocks, T, max_q, hq, hkv, n_split, scale, 0, 0, ksc, vsc, st);
     if (rc) return rc;
-    if ((rc = s.linear(o, hq * 128, ptr(4), H, h, x))) return rc;
-    if ((rc = pm_rmsnorm_fwd(h, nullptr, ptr(5), y, nullptr, rstd, T, H, eps, st))) return rc;
-    if (T <= kSkinnyRows) {
-      if ((rc = pm_linear_skinny(y, H, ptr(6), H, act, I, nullptr, 0, T, I, H, 1, 1.f, 0, 1, status, st))) return rc;
-    } else {
-      if ((rc = s.linear(y, H, ptr(6), 2 * I, gu, nullptr))) return rc;
-      if ((rc = pm_swiglu_fwd(gu, act, T, I, st))) return rc;
-    }
     void* to = l == n_layers - 1 ? out : xa;
-    if ((rc = s.linear(act, I, ptr(7), H, to, h))) return rc;
+    if (few) {
+      const void* next = l == n_layers - 1 ? nullptr : reinterpret_cast<void*>(p[12]);      // the next layer's input norm
+      if ((rc = s.residual(o, hq * 128, ptr(4), H, h, x, ptr(5), y, rstd))) return rc;
+      if ((rc = s.normed(y, rstd, parts, H, ptr(6), I, act, 1))) return rc;
+      if ((rc = s.residual(act, I, ptr(7), H, to, h, next, y, rstd))) return rc;
+    } else {
+      if ((rc = s.tile(o, hq * 128, ptr(4), H, h, x))) return rc;
+      if ((rc = pm_rmsnorm_fwd(h, nullptr, ptr(5), y, nullptr, rstd, T, H, eps, st))) return rc;
+      if ((rc = s.tile(y, H, ptr(6), 2 * I, gu, nullptr))) return rc;
+      if ((rc = pm_swiglu_fwd(gu, act, T, I, st))) return rc;
+      if ((rc = s.tile(act, I, ptr(7), H, to, h))) return rc;
+    }
     x = to;
   }
   return 0;

@@ -199,12 +199,20 @@ int pm_gemm_q4_2sm(const void* A, int lda, int a_rows, const void* codes, const 
     int* status, cudaStream_t stream);
 
 // ---------------------------------------------------------------- gemm_skinny.cu
+// pm_linear_skinny inside a chain of RMSNorms. ss_in non-null: x is rows * norm weight and ss_in [parts_in][128] their partial sums of squares
+// (row m of part i at i * 128 + m), the product is that of the normalised rows. y2 non-null (not with swiglu): y2 = y * nw_out with y's
+// strides and ss_out [(N + 127) / 128][128] for the next link.
+int pm_linear_skinny_norm(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy, const
+    void* res, long long ldr, int M, int N, int K, int swiglu, float alpha, int splits, int chain, const float*
+    ss_in, int parts_in, float eps, const void* nw_out, void* y2, float* ss_out, int* status, cudaStream_t st);
 // x: [M, K] rows ldx apart, w: [N, K] (swiglu: [2 N, K], gate rows first) rows ldw apart, y / res: [M, N] rows ldy / ldr apart (res
 // nullable, may be y). M <= 128; K, N and the row strides multiples of 8, pointers 16-byte aligned. splits 0: chosen here. chain: see
 // the head of this file. Returns a negative value for arguments outside of that.
 int pm_linear_skinny(const void* x, long long ldx, const void* w, long long ldw, void* y, long long ldy, const
     void* res, long long ldr, int M, int N, int K, int swiglu, float alpha, int splits, int chain, int* status,
     cudaStream_t st);
+// First link of such a chain: y2 = x * nw [M, H] and ss [128] = the rows' sums of squares. M <= 128, H a multiple of 8.
+int pm_skinny_prep(const void* x, const void* nw, void* y2, float* ss, int M, int H, cudaStream_t st);
 
 // ---------------------------------------------------------------- gemm_tcgen05.cu
 // Returns 0 on success, negative on argument / descriptor errors, or the CUDA error code.

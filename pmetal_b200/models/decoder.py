@@ -461,7 +461,7 @@ class DecoderLM(nn.Module):
         if (skinny and not return_hidden and x.shape[0] <= GEMV_MAX_ROWS and cfg.final_logit_softcap <= 0
                 and head.dtype == torch.bfloat16 and not head.requires_grad):
             from ..ops import native as nat
-            return nat.gemv(x.contiguous(), head, self.norm, cfg.rms_norm_eps)      # final norm fused into the head
+            return nat.few_row_head(x.contiguous(), head, self.norm, cfg.rms_norm_eps)
         x = ops.rms_norm(x, self.norm, cfg.rms_norm_eps)
         return x if return_hidden else self.logits(x)
 

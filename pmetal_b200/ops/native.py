@@ -211,6 +211,32 @@ def raw_gemm(A, a_mn, lda, a_rows, B, b_mn, ldb, b_rows, D, out_mode, ldd, M, N,
     _chk(rc, "pm_gemm_bf16")
 
 
+def _skinny(x, w, out, residual, alpha: float = 1.0) -> bool:
+    """out = alpha x w^T (+ residual) by the few-row kernel (csrc/gemm_skinny.cu) where that is the faster one; False where it is not or its
+    alignment rules do not hold. Measured (it, the tile GEMM) in us at K = 1024 to 3072: 64 rows x 4096 columns 7.5, 7.9, x 1024 7.2, 9.6;
+    128 rows x 4096 columns 9.3, 7.9, x 1024 8.5, 10.9: above 64 rows only where there are few column tiles."""
+    M, K = x.shape
+    N = w.shape[0]
+    if M > 128 or (M > 64 and -(-N // 128) * 8 > sm_count()) or (N | K) % 8 or TUNA:
+        return False
+    ts = (x, w, out) if residual is None else (x, w, out, residual)
+    if any(t.stride(0) % 8 or t.stride(1) != 1 or t.data_ptr() % 16 or t.dtype != torch.bfloat16 for t in ts):
+        return False
+    _chk(lib().pm_linear_skinny(_p(x), c_ll(x.stride(0)), _p(w), c_ll(w.stride(0)), _p(out), c_ll(out.stride(0)), _p(residual),
+                                c_ll(residual.stride(0) if residual is not None else 0), c_int(M), c_int(N), c_int(K), c_int(0),
+                                c_float(alpha), c_int(0), c_int(0), _p(status_word(x.device)), _stream()), "pm_linear_skinny")
+    return True
+
+
+def few_row_head(x, head, norm_w, eps: float):
+    """Logits of a few rows: final norm and output projection."""
+    h = rmsnorm_fwd(x, norm_w, eps)[1]
+    out = torch.empty(x.shape[0], head.shape[0], dtype=torch.bfloat16, device=x.device)
+    if _skinny(h, head, out, None):
+        return out
+    return gemv(x, head, norm_w, eps)
+
+
 SPLIT_K = os.environ.get("PMETAL_GEMM_SPLITK", "1") == "1"
 FUSED_Q4 = os.environ.get("PMETAL_FUSED_Q4", "0") == "1"      # opt-in: saves the transient bf16 weight, not time
 _SPLITK_WS = {}
@@ -248,6 +274,8 @@ def gemm(x: torch.Tensor, w: torch.Tensor, alpha: float = 1.0, residual: Optiona
     Nw = max(N, pad_n_to)
     if out is None:
         out = torch.empty(M, Nw, dtype=torch.bfloat16, device=x.device)
+    if not bn and Nw == N and _skinny(x, w, out, residual, alpha):
+        return out
 
     def run(b):
         raw_gemm(x, 0, x.stride(0), M, w, 0, w.stride(0), N, out, 0, out.stride(0), M, Nw, K, R=residual,
@@ -265,6 +293,8 @@ def gemm_lora(x, w, t, b, seg_sizes, r, residual=None, bn: int = 0) -> torch.Ten
     M, K = x.shape
     N = w.shape[0]
     out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
+    if t is None and not bn and _skinny(x, w, out, residual):
+        return out
     bn = bn or _pick_bn(N, seg_sizes, M)
     kw = {}
     if t is not None:
@@ -908,7 +938,7 @@ def layer_stack(rows, x, meta, cos, sin, hq: int, hkv: int, inter: int, num_bloc
     scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
     out = torch.empty_like(x)
     global LAUNCHES
-    LAUNCHES += n_layers * (8 if T <= 128 else 9) - 1
+    LAUNCHES += n_layers * (6 if T <= 128 else 9)
     _chk(lib().pm_layer_stack((c_ll * len(rows))(*rows), c_int(n_layers), _p(x), _p(out), _p(scratch), c_ll(nbytes), c_int(T), c_int(H),
                               c_int(hq), c_int(hkv), c_int(inter), c_float(eps), c_float(scale), _p(cos), _p(sin), _p(meta.slots),
                               _p(meta.block_table), _p(meta.seq_lens), _p(meta.q_start), _p(meta.q_lens), c_int(n_seq),

@@ -89,3 +89,21 @@ def test_layer_stack_leaves_other_models_alone():
     m = make()
     apply_lora(m, LoraConfig(r=8, alpha=8, target_modules=["q_proj"]), seed=0)
     assert m._stack_addresses(m.new_cache(4)) is None
+
+
+@pytest.mark.parametrize("M,N", [(16, 4096), (64, 24), (65, 4096), (65, 1024), (128, 136)])
+def test_gemm_on_few_rows_takes_either_kernel(M, N):
+    """Strided operands and results, with and without a residual, on both sides of the rule that picks the few-row kernel."""
+    from pmetal_b200.ops import native as nat
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, 776, device="cuda", generator=g).to(torch.bfloat16)[:, :768]
+    w = (torch.randn(N, 768, device="cuda", generator=g) * 768 ** -0.5).to(torch.bfloat16)
+    res = torch.randn(M, N, device="cuda", generator=g).to(torch.bfloat16)
+    want = x.float() @ w.float().t()
+    assert _rel(nat.gemm(x, w), want) < 3e-3 and _rel(nat.gemm(x, w, residual=res), want + res.float()) < 3e-3
+    assert _rel(nat.gemm_lora(x, w, None, None, (N,), 0, res), want + res.float()) < 3e-3
+    h = torch.randn(3, 768, device="cuda", generator=g).to(torch.bfloat16)
+    nw = torch.rand(768, device="cuda", generator=g).to(torch.bfloat16)
+    normed = h.float() * torch.rsqrt(h.float().square().mean(-1, keepdim=True) + 1e-6) * nw.float()
+    assert _rel(nat.few_row_head(h, w, nw, 1e-6), normed @ w.float().t()) < 5e-3
+    nat.check_status()
