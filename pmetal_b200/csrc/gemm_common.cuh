@@ -27,7 +27,7 @@ struct GemmParams {
   float alpha;
   void* D;
   const void* R;
-  int seg_mode;    // 0 none; 1: A2 K-offset = seg(n0)*seg_r; 2: B mn-offset = seg(m0)*seg_r; 3: B mn-offset = -seg(k)*seg_r
+  int seg_mode;    // 0 none; 1: A2 K-offset = seg(n0)*seg_r; 2: B mn-offset = seg(m0)*seg_r
   int seg_end[4];
   int seg_r;
   int tmem_cols;

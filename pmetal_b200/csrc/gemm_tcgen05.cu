@@ -102,11 +102,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             uint8_t* sa = smem + s * stage_bytes;
             mbar_expect_tx(&full_bar[s], stage_bytes);
             load_operand(sa, ma, &full_bar[s], amn, kBM, m0, ka);
-            // seg_mode 3: B is [K, seg_r] (MN-major, one narrow block of columns shared by every segment of K); the
-            // tile is fetched seg * seg_r columns to the left of its origin, so the rows of segment `seg` land in
-            // output columns [seg * seg_r, (seg + 1) * seg_r) and everything else reads as zero (out-of-range fill)
-            const int shift = (!part && p.seg_mode == 3) ? seg_of(p, kbk) * p.seg_r : 0;
-            load_operand(sa + a_bytes, mbp, &full_bar[s], bmn, p.bn, brow - shift, kbk);
+            load_operand(sa + a_bytes, mbp, &full_bar[s], bmn, p.bn, brow, kbk);
           }
           ka += kBK;
           kbk += kBK;
@@ -288,8 +284,6 @@ extern "C" int pm_gemm_bf16(const void* A, int a_mn, int lda, int a_rows, const 
   if (M <= 0 || N <= 0 || K <= 0) return -13;
   if ((out_mode == 0 || out_mode == 6) && ((ldd % 8) || (reinterpret_cast<uintptr_t>(D) & 15))) return -14;
   if (R && ((ldr % 8) || (reinterpret_cast<uintptr_t>(R) & 15))) return -15;
-  // seg_mode 3 shifts a TMA load by seg * seg_r elements: the shift must keep the 16-byte alignment of the copy
-  if (seg_mode == 3 && (!b_mn || (seg_r % 8) || N > bn || splits != 1)) return -16;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.K2 = K2; p.bn = bn;
   p.a_mn = a_mn; p.b_mn = b_mn; p.a2_mn = a2_mn; p.b2_mn = b2_mn;

@@ -305,8 +305,24 @@ def gemm_lora(x, w, t, b, seg_sizes, r, residual=None, bn: int = 0) -> torch.Ten
     return out
 
 
+def _lora_tall(x, b, b_mn: int, nr: int, seg_sizes, scale: float) -> Optional[torch.Tensor]:
+    """[M, 64] product with a narrow factor by csrc/lora_tall.cu, or None outside of its rules."""
+    M, K = x.shape
+    if nr % 8 or K % 8 or x.stride(0) % 8 or x.stride(1) != 1 or not b.is_contiguous() or (x.data_ptr() | b.data_ptr()) % 16:
+        return None
+    out = torch.empty(M, 64, dtype=torch.bfloat16, device=x.device)
+    _chk(lib().pm_lora_tall(_p(x), c_ll(x.stride(0)), _p(b), c_ll(b.stride(0)), c_int(b_mn), c_int(nr), _p(out), c_ll(64), c_int(M), c_int(K),
+                            _seg_ends(seg_sizes) if len(seg_sizes) > 1 else None, c_float(scale), c_int(0), _p(status_word(x.device)),
+                            _stream()), "pm_lora_tall")
+    return out
+
+
 def lora_t(x, a, scale: float) -> torch.Tensor:
     """t = scale * x a^T, padded to a multiple of 64 columns (padding is zero)."""
+    if a.shape[0] <= 64:
+        t = _lora_tall(x, a, 0, a.shape[0], (), scale)
+        if t is not None:
+            return t
     return gemm(x, a, alpha=scale, pad_n_to=_t_width(a.shape[0]), bn=64)
 
 
@@ -314,14 +330,11 @@ def lora_dt(dy, b, seg_sizes, r, scale) -> torch.Tensor:
     """dt[:, seg*r:(seg+1)*r] = scale * dy[:, seg] b_seg   ([M, 64-padded]); padding columns are unspecified."""
     M, N = dy.shape
     nseg = len(seg_sizes)
+    if MN_MAJOR and nseg * r <= 64 and nseg <= 4 and all(s % 64 == 0 for s in seg_sizes) and b.shape[1] == r:
+        dt = _lora_tall(dy, b, 1, r, seg_sizes, scale)
+        if dt is not None:
+            return dt
     dt = torch.empty(M, _t_width(nseg * r), dtype=torch.bfloat16, device=dy.device)
-    if (MN_MAJOR and nseg * r <= 64 and r % 8 == 0 and all(s % 64 == 0 for s in seg_sizes) and b.is_contiguous()
-            and b.shape[1] == r):
-        # one launch: b [N, r] is read in place as an MN-major operand; segment s of the reduction lands in output
-        # columns [s r, (s + 1) r) because its tile is fetched s r columns left of the origin (zero fill elsewhere)
-        raw_gemm(dy, 0, dy.stride(0), M, b, 1, r, r, dt, 0, dt.stride(0), M, 64, N, alpha=scale, bn=64,
-                 seg_mode=3, seg_sizes=seg_sizes, seg_r=r)
-        return dt
     b_t = b.t().contiguous()                      # [r, N], K-major over N
     n0 = 0
     for i, sz in enumerate(seg_sizes):
