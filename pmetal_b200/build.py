@@ -34,7 +34,7 @@ COMPONENTS = {
     "ravapel": ("attention_tc", "gated_linear", "gemm_2sm", "gemm_skinny", "gemm_tcgen05", "gemv", "linear_attn", "postnorm", "sandwich", "ssd_chunk",
                 "window_attn"),
     "decoder": ("attention", "attention_tc", "elementwise", "gemm_2sm", "gemm_skinny", "gemm_tcgen05", "gemv", "grouped_gemm",
-                "layer_stack", "lora_tall", "moe_quant", "paged_decode"),
+                "layer_stack", "lora_linear", "lora_tall", "moe_quant", "paged_decode"),
 }
 
 

@@ -323,6 +323,26 @@ int pm_norm_gate(const void* y, const void* gate, int f32, long long ldg, const 
     width, int silu, void* out, int n_tok, const float* den, int shared, float scale, long long ldo, cudaStream_t
     st);
 
+// ---------------------------------------------------------------- lora_linear.cu
+// t = scale x a^T [M, 64], y = x w^T + t[:, segment] b_segment^T (+ residual). x: [M, K] rows ldx apart, w: [N, K] rows ldw apart, a: [nseg r, K],
+// b: [N, r], y: [M, N], residual (nullable) rows ldr apart. bn: tile width; M > 128.
+int pm_lora_linear_fwd(const void* x, int ldx, const void* w, int ldw, const void* a, const void* b, const void*
+    residual, int ldr, void* t, void* y, int M, int N, int K, const int* seg_end, int nseg, int r, float scale, int
+    bn, int* status, cudaStream_t st);
+// dt = scale dy b [M, 64], dx = dy w + dt a (dx null: left out), ga [nseg r, K] += dt^T x, gb [N, r] += dy^T t, both fp32. w: [N, K] (w_t 0) or its
+// transpose [K, N] (w_t 1), rows ldw apart; bn: tile width of dx.
+int pm_lora_linear_bwd(const void* dy, int ldd, const void* w, int w_t, int ldw, const void* a, const void* b,
+    const void* x, int ldx, const void* t, void* dt, void* dx, float* ga, float* gb, int M, int N, int K, const
+    int* seg_end, int nseg, int r, float scale, int bn, int* status, cudaStream_t st);
+
+// ---------------------------------------------------------------- lora_tall.cu
+// x: [M, K] rows ldx apart. b_mn 0: b is [nr, K] rows ldb apart and d = alpha x b^T; b_mn 1: b is [K, nr], d[:, seg nr ..] = alpha x[:, seg] b[seg]
+// with the cumulative ends of the segments in seg_end[4] (multiples of 64; 0x7fffffff beyond the last but one). d: [M, 64] rows ldd apart, all 64 columns
+// are written (zeros beyond the factors). nr and segments * nr up to 64, multiples of 8; K, the row strides multiples of 8, pointers
+// 16-byte aligned. splits 0: chosen here.
+int pm_lora_tall(const void* x, long long ldx, const void* b, long long ldb, int b_mn, int nr, void* d, long long
+    ldd, int M, int K, const int* seg_end, float alpha, int splits, int* status, cudaStream_t st);
+
 // ---------------------------------------------------------------- mhc.cu
 // x [T, n, C] bf16; either phi [n C, n^2 + 2n] fp32 (dot products formed here) or raw [T, ld_raw] fp32 = x . phi computed by
 // the caller; bias [n^2 + 2n], alpha [3]; n in {2, 4, 8}, C % 8 == 0, iters <= 32.

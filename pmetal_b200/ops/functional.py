@@ -343,11 +343,14 @@ class _LoraLinearFn(torch.autograd.Function):
             # QLoRA off the fused shapes: dequantise into a transient buffer; only the packed weight is kept
             from ..lora.qlora import dequantize_weight
             w, w_t = dequantize_weight(qweight), None
-        t = nat.lora_t(x, a, scale) if a is not None else None    # [M, 64-padded] = s x A^T
+        t = None                                                  # [M, 64-padded] = s x A^T
         if fused_q:       # the GEMM expands the 4-bit codes on their way into the tensor cores
+            t = nat.lora_t(x, a, scale) if a is not None else None
             y = nat.gemm_q4_lora(x, qweight, t, b, seg_sizes, r, residual)
+        elif a is not None:
+            t, y = nat.lora_linear_fwd(x, w, a, b, seg_sizes, r, scale, residual)
         else:
-            y = nat.gemm_lora(x, w, t, b, seg_sizes, r, residual)
+            y = nat.gemm_lora(x, w, None, b, seg_sizes, r, residual)
         ctx.fused_q = fused_q
         ctx.save_for_backward(x, None if qweight is not None else w, w_t, a, b, t)
         ctx.params = (a32, b32)
@@ -368,10 +371,6 @@ class _LoraLinearFn(torch.autograd.Function):
         dy = dy.contiguous()
         da = db = dx = None
         if a is not None:
-            dt = nat.lora_dt(dy, b, seg_sizes, r, scale)          # [M, 64-padded] = s dY_seg B_seg
-            if ctx.needs_input_grad[0]:
-                dx = nat.gemm_q4_lora_dx(dy, ctx.qweight, dt, a) if fused_q else nat.gemm_lora_dx(dy, w, w_t, dt, a)
-
             def target(p32):
                 g = p32.grad
                 if g is not None and g.dtype == torch.float32 and g.is_contiguous():
@@ -380,8 +379,14 @@ class _LoraLinearFn(torch.autograd.Function):
                 return z, z
             ga, da = target(a32)
             gb, db = target(b32)
-            nat.lora_da(dt, x, a.shape[0], ga)
-            nat.lora_db(dy, t, seg_sizes, r, gb)
+            if fused_q:
+                dt = nat.lora_dt(dy, b, seg_sizes, r, scale)      # [M, 64-padded] = s dY_seg B_seg
+                if ctx.needs_input_grad[0]:
+                    dx = nat.gemm_q4_lora_dx(dy, ctx.qweight, dt, a)
+                nat.lora_da(dt, x, a.shape[0], ga)
+                nat.lora_db(dy, t, seg_sizes, r, gb)
+            else:
+                dx = nat.lora_linear_bwd(dy, w, w_t, a, b, x, t, seg_sizes, r, scale, ga, gb, ctx.needs_input_grad[0])
         elif ctx.needs_input_grad[0]:
             dx = nat.gemm_q4_lora_dx(dy, ctx.qweight, None, None) if fused_q else nat.gemm_lora_dx(dy, w, w_t, None, None)
         return dx, None, None, da, db, None, None, None, None, None, (dy if has_res else None), None

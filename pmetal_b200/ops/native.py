@@ -344,6 +344,72 @@ def lora_dt(dy, b, seg_sizes, r, scale) -> torch.Tensor:
     return dt
 
 
+_LORA_ARGS = {}
+
+
+def _lora_call(name: str, spec: str, *args) -> None:
+    """``lib().name(*args)``; ``spec`` gives the argument types once (p pointer, i int, f float), so that a call converts none itself."""
+    fn = _LORA_ARGS.get(name)
+    if fn is None:
+        fn = getattr(lib(), name)
+        fn.restype, fn.argtypes = c_int, [{"p": c_void_p, "i": c_int, "f": c_float}[c] for c in spec]
+        _LORA_ARGS[name] = fn
+    _chk(fn(*args), name)
+
+
+def _lora_fused_ok(x, a, b, seg_sizes, r: int, *more) -> bool:
+    """Whether a layer's narrow and wide products run from one call (csrc/lora_linear.cu): the rules of csrc/lora_tall.cu and of the GEMMs."""
+    n = len(seg_sizes)
+    return (MN_MAJOR and not TUNA and not DETERMINISTIC and x.shape[0] > 128 and r % 8 == 0 and n * r <= 64 and n <= 4
+            and all(s % 128 == 0 for s in seg_sizes[:-1]) and seg_sizes[-1] % 64 == 0 and x.shape[1] % 8 == 0 and a.shape[0] == n * r and b.shape[1] == r
+            and a.is_contiguous() and b.is_contiguous() and (a.data_ptr() | b.data_ptr()) % 16 == 0
+            and all(t.dtype == torch.bfloat16 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (x, *more)))
+
+
+def lora_linear_fwd(x, w, a, b, seg_sizes, r: int, scale: float, residual=None):
+    """(t, y) of a LoRA layer: ``lora_t`` and ``gemm_lora``, issued by one call where the shapes allow."""
+    more = (w,) if residual is None else (w, residual)
+    if not _lora_fused_ok(x, a, b, seg_sizes, r, *more):
+        t = lora_t(x, a, scale)
+        return t, gemm_lora(x, w, t, b, seg_sizes, r, residual)
+    M, K = x.shape
+    N = w.shape[0]
+    t = torch.empty(M, 64, dtype=torch.bfloat16, device=x.device)
+    y = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
+    global LAUNCHES
+    LAUNCHES += 1
+    _lora_call("pm_lora_linear_fwd", "pipipppippiiipiifipp", x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), a.data_ptr(), b.data_ptr(),
+               residual.data_ptr() if residual is not None else 0, residual.stride(0) if residual is not None else 0, t.data_ptr(),
+               y.data_ptr(), M, N, K, _seg_ends(seg_sizes), len(seg_sizes), r, scale, _pick_bn(N, seg_sizes, M),
+               status_word(x.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+    return t, y
+
+
+def lora_linear_bwd(dy, w, w_t, a, b, x, t, seg_sizes, r: int, scale: float, ga, gb, want_dx: bool):
+    """dx (or None) of a LoRA layer; adds the factors' gradients to ``ga`` and ``gb`` (fp32). ``lora_dt``, ``gemm_lora_dx``, ``lora_da`` and
+    ``lora_db``, issued by one call where the shapes allow."""
+    wide = w_t if w_t is not None else w
+    if (not _lora_fused_ok(dy, a, b, seg_sizes, r, x, wide) or x.shape[1] % 8 or t.shape[1] != 64 or not t.is_contiguous()
+            or not (ga.is_contiguous() and gb.is_contiguous())):
+        dt = lora_dt(dy, b, seg_sizes, r, scale)                  # [M, 64-padded] = s dY_seg B_seg
+        dx = gemm_lora_dx(dy, w, w_t, dt, a) if want_dx else None
+        lora_da(dt, x, a.shape[0], ga)
+        lora_db(dy, t, seg_sizes, r, gb)
+        return dx
+    M, N = dy.shape
+    K = x.shape[1]
+    dt = torch.empty(M, 64, dtype=torch.bfloat16, device=dy.device)
+    dx = torch.empty(M, K, dtype=torch.bfloat16, device=dy.device) if want_dx else None
+    bn = _pick_bn(K)
+    global LAUNCHES
+    LAUNCHES += 3 if want_dx else 2
+    _lora_call("pm_lora_linear_bwd", "pipiipppipppppiiipiifipp", dy.data_ptr(), dy.stride(0), wide.data_ptr(), int(w_t is not None),
+               wide.stride(0), a.data_ptr(), b.data_ptr(), x.data_ptr(), x.stride(0), t.data_ptr(), dt.data_ptr(),
+               dx.data_ptr() if want_dx else 0, ga.data_ptr(), gb.data_ptr(), M, N, K, _seg_ends(seg_sizes), len(seg_sizes), r, scale,
+               bn if w_t is not None else max(bn, 64), status_word(dy.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+    return dx
+
+
 def gemm_lora_dx(dy, w, w_t, dt, a) -> torch.Tensor:
     """dx = dy w (+ dt[:, :nr] a).  w:[N,K_in]; w_t:[K_in,N] optional; a:[nr,K_in]."""
     M, N = dy.shape
@@ -463,6 +529,17 @@ def lora_db(dy, t, seg_sizes, r: int, out: torch.Tensor) -> None:
         return
     nk = -(-M // 64)
     det = DETERMINISTIC
+    if any(s % 128 for s in seg_sizes[:-1]):       # a 128-row tile of the launch below would straddle two segments
+        n0 = 0
+        for i, sz in enumerate(seg_sizes):
+            d, ti, o = dy[:, n0:n0 + sz], t[:, i * r:], out[n0:n0 + sz]
+            if (d.data_ptr() | ti.data_ptr()) % 16:
+                o.add_(d.t().float() @ ti[:, :r].float())
+            else:
+                raw_gemm(d, 1, dy.stride(0), sz, ti, 1, t.stride(0), t.shape[1] - i * r, o, 4 if det else 2, out.stride(0), sz, 64, M,
+                         n_store=r, bn=64, splits=1 if det else _splits_for(-(-sz // 128), nk))
+            n0 += sz
+        return
     raw_gemm(dy, 1, dy.stride(0), N, t, 1, t.stride(0), t.shape[1], out, 4 if det else 2, out.stride(0), N, 64, M,
              n_store=r, bn=64, splits=1 if det else _splits_for(-(-N // 128), nk),
              seg_mode=2 if len(seg_sizes) > 1 else 0, seg_sizes=seg_sizes, seg_r=r)

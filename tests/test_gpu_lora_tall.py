@@ -46,3 +46,28 @@ def test_other_ranks_keep_the_general_path():
         for i, n in enumerate(segs):
             assert _rel(got[:, i * r:(i + 1) * r], 2 * dy[:, at:at + n].float() @ b[at:at + n].float()) < 3e-3, (r, i)
             at += n
+
+
+@pytest.mark.parametrize("M", [100, 129, 300, 1537])
+@pytest.mark.parametrize("segs,r,K", [((256, 128, 128), 16, 256), ((192,), 16, 136), ((64, 64), 32, 520), ((64, 128), 16, 64)])
+@pytest.mark.parametrize("transposed", [True, False])
+def test_lora_layer_in_one_call(M, segs, r, K, transposed):
+    """Forward and gradients of a layer through the one-call entries and, outside of their rules, through the single products."""
+    from pmetal_b200.ops import functional as ops
+    g = torch.Generator(device="cuda").manual_seed(M + K + r)
+    N, nr = sum(segs), r * len(segs)
+    f = lambda *s: torch.randn(*s, device="cuda", generator=g)      # noqa: E731
+    x, res, dy = f(M, K).to(torch.bfloat16).requires_grad_(True), f(M, N).to(torch.bfloat16), f(M, N).to(torch.bfloat16)
+    w = (f(N, K) * K ** -0.5).to(torch.bfloat16)
+    a, b = (f(nr, K) * K ** -0.5).requires_grad_(True), (f(N, r) * 0.1).requires_grad_(True)
+    y = ops.lora_linear(x, w, w.t().contiguous() if transposed else None, a, b, segs, r, 2.0, res)
+    got = torch.autograd.grad(y, (x, a, b), dy)
+    xr, ar, br = (t.detach().to(torch.bfloat16).float().requires_grad_(True) for t in (x, a, b))
+    parts, at = [], 0
+    for i, n in enumerate(segs):
+        parts.append(2.0 * (xr @ ar[i * r:(i + 1) * r].t()) @ br[at:at + n].t())
+        at += n
+    want = xr @ w.float().t() + res.float() + torch.cat(parts, -1)
+    assert _rel(y.detach(), want.detach()) < 4e-3                    # bf16 t and y
+    for p, q in zip(got, torch.autograd.grad(want, (xr, ar, br), dy.float())):
+        assert _rel(p, q) < 6e-3                                     # bf16 dt, t and dx
