@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kMhcThreads) mhc_post_res_kernel(const __nv_bf
 
 // ---------------------------------------------------------------------------------------------- stream mixing (backward)
 // Either half may be absent (null dh_in: only the post / res part; null dx_out: only the pre part), since autograd reaches
-// the two applications at different times.
+// the two applications at different times. The gains of an absent half are not read (they may be null).
 // dx[t, n] = H_pre[t, n] dh_in[t] + sum_m H_res[t, m, n] dx_out[t, m];  dh_out[t] = sum_m H_post[t, m] dx_out[t, m]
 // dH_pre[t, n] = <x[t, n], dh_in[t]>;  dH_post[t, m] = <dx_out[t, m], h_out[t]>;  dH_res[t, m, n] = <dx_out[t, m], x[t, n]>
 template <int N>
@@ -230,8 +230,11 @@ __global__ void __launch_bounds__(kMhcThreads) mhc_mix_bwd_kernel(const __nv_bfl
   __shared__ float red[(kMhcThreads / 32) * CNT];
   __shared__ float tot[CNT];
   const long long t = blockIdx.x;
-  if (threadIdx.x < N * N) sr[threadIdx.x] = h_res[t * N * N + threadIdx.x];
-  if (threadIdx.x < N) { sp[threadIdx.x] = h_post[t * N + threadIdx.x]; sq[threadIdx.x] = h_pre[t * N + threadIdx.x]; }
+  if (threadIdx.x < N * N) sr[threadIdx.x] = dx_out ? h_res[t * N * N + threadIdx.x] : 0.f;
+  if (threadIdx.x < N) {
+    sp[threadIdx.x] = dx_out ? h_post[t * N + threadIdx.x] : 0.f;
+    sq[threadIdx.x] = dh_in ? h_pre[t * N + threadIdx.x] : 0.f;
+  }
   __syncthreads();
   float acc[CNT];          // [pre n | post m | res m*N + n]
 #pragma unroll
@@ -443,6 +446,7 @@ extern "C" int pm_mhc_mix_bwd(const void* x, const void* h_out, const void* dh_i
                               const float* h_post, const float* h_res, int T, int n, int C, void* dx, void* dh_out,
                               float* d_pre, float* d_post, float* d_res, cudaStream_t st) {
   if (T <= 0 || (C % 8)) return -2;
+  if ((dh_in && (!h_pre || !d_pre)) || (dx_out && (!h_out || !h_post || !h_res || !dh_out || !d_post || !d_res))) return -3;
   MHC_DISPATCH(n, (mhc_mix_bwd_kernel<NN><<<T, kMhcThreads, 0, st>>>(
                       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(h_out),
                       static_cast<const __nv_bfloat16*>(dh_in), static_cast<const __nv_bfloat16*>(dx_out), h_pre, h_post,

@@ -659,12 +659,9 @@ def mhc_mix_bwd(x, h_out, dh_in, dx_out, h_pre, h_post, h_res):
     dh_out = torch.empty(T, C, dtype=x.dtype, device=x.device) if dx_out is not None else None
     d_pre = f(T, n) if dh_in is not None else None
     d_post, d_res = (f(T, n), f(T, n, n)) if dx_out is not None else (None, None)
-    dummy = torch.zeros(n * n, dtype=torch.float32, device=x.device)          # unused halves still need readable gains
     lib().pm_mhc_mix_bwd.restype = c_int
-    _chk(lib().pm_mhc_mix_bwd(_p(x), _p(h_out), _p(dh_in), _p(dx_out), _p(h_pre if h_pre is not None else dummy),
-                              _p(h_post if h_post is not None else dummy), _p(h_res if h_res is not None else dummy),
-                              c_int(T), c_int(n), c_int(C), _p(dx), _p(dh_out), _p(d_pre), _p(d_post), _p(d_res),
-                              _stream()), "pm_mhc_mix_bwd")
+    _chk(lib().pm_mhc_mix_bwd(_p(x), _p(h_out), _p(dh_in), _p(dx_out), _p(h_pre), _p(h_post), _p(h_res), c_int(T), c_int(n),
+                              c_int(C), _p(dx), _p(dh_out), _p(d_pre), _p(d_post), _p(d_res), _stream()), "pm_mhc_mix_bwd")
     return dx, dh_out, d_pre, d_post, d_res
 
 

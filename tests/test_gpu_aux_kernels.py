@@ -598,3 +598,28 @@ def test_hyper_connection_kernels(n, C):
     xe = (torch.randn(50, C, device="cuda")).bfloat16()
     assert torch.equal(mhc.expand_streams(xe, n)[:, n - 1], xe)
     _close(mhc.collapse_streams(x), x.float().mean(1), what="collapse")
+
+
+@pytest.mark.parametrize("n,C", [(4, 256), (8, 64)])
+def test_hyper_connection_gradient_of_one_half(n, C):
+    """Each half of the stream gradients alone, with NaN in the memory that small allocations get: what belongs to the absent half is
+    not read."""
+    nat = _nat()
+    torch.manual_seed(3)
+    T = 300
+    x = torch.randn(T, n, C, device="cuda").bfloat16()
+    h_out, dh_in = torch.randn(T, C, device="cuda").bfloat16(), torch.randn(T, C, device="cuda").bfloat16()
+    dy = torch.randn(T, n, C, device="cuda").bfloat16()
+    pre, post, res = torch.rand(T, n, device="cuda"), torch.rand(T, n, device="cuda"), torch.rand(T, n, n, device="cuda")
+    poison = [torch.full((k,), float("nan"), device="cuda") for k in (64, 128, 1 << 12, 1 << 17) for _ in range(64)]
+    del poison
+    dx, dh, d_pre, d_post, d_res = nat.mhc_mix_bwd(x, None, dh_in, None, pre, None, None)
+    assert dh is None and d_post is None and d_res is None
+    _close(dx, pre[:, :, None] * dh_in.float()[:, None], what="dx of the read half")
+    _close(d_pre, torch.einsum("tnc,tc->tn", x.float(), dh_in.float()), what="dH_pre")
+    dx, dh, d_pre, d_post, d_res = nat.mhc_mix_bwd(x, h_out, None, dy, None, post, res)
+    assert d_pre is None
+    _close(dx, torch.einsum("tmn,tmc->tnc", res, dy.float()), what="dx of the write half")
+    _close(dh, torch.einsum("tm,tmc->tc", post, dy.float()), what="dh_out")
+    _close(d_post, torch.einsum("tmc,tc->tm", dy.float(), h_out.float()), what="dH_post")
+    _close(d_res, torch.einsum("tmc,tnc->tmn", dy.float(), x.float()), what="dH_res")

@@ -109,3 +109,29 @@ def test_gguf_reader_survives_mutated_files():
 
     mutate()
     garbage()
+
+
+@pytest.mark.parametrize("read_half", [True, False])
+def test_stream_gradient_of_one_half_passes_nothing_for_the_other(monkeypatch, read_half):
+    """The gains of an absent half are per token, so a stand-in of another size would be read out of range: they are null."""
+    from pmetal_b200.ops import native
+    calls = []
+
+    class Lib:
+        class pm_mhc_mix_bwd:
+            restype = None
+
+            def __new__(cls, *args):
+                calls.append(args)
+                return 0
+    monkeypatch.setattr(native, "lib", lambda: Lib)
+    monkeypatch.setattr(native, "_stream", lambda: native.c_void_p(0))
+    x, h, dy = torch.zeros(5, 4, 8), torch.zeros(5, 8), torch.zeros(5, 4, 8)
+    pre, post, res = torch.zeros(5, 4), torch.zeros(5, 4), torch.zeros(5, 4, 4)
+    if read_half:
+        native.mhc_mix_bwd(x, None, h, None, pre, None, None)
+    else:
+        native.mhc_mix_bwd(x, h, None, dy, None, post, res)
+    h_out, dh_in, dx_out, h_pre, h_post, h_res = (a.value for a in calls[0][1:7])
+    assert (dh_in is not None) == (h_pre is not None) == read_half
+    assert (dx_out is None) == (h_out is None) == (h_post is None) == (h_res is None) == read_half
