@@ -239,7 +239,7 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       const int col_base = nb * kBN;
       const uint32_t tm = tmem_base + buf * kBN + (static_cast<uint32_t>(q * 32) << 16);
       if (staged) {
-        const int pieces = row0 < p.M ? min(kBN / 64, (p.n_store - col_base + 63) / 64) : 0;
+        const int pieces = row0 < p.M ? max(0, min(kBN / 64, (p.n_store - col_base + 63) / 64)) : 0;   // none past n_store
         if (p.R && lane == 0) {
           tma_store_wait_read<0>();
           for (int c = 0; c < min(2, pieces); ++c) {

@@ -43,3 +43,19 @@ def test_pair_gemm_tile_edges(M, N, K, segs):
             at += n
         _near(nat.gemm_lora(x, w, t, b, segs, 16, res), want, "segments")
     nat.check_status()
+
+
+# tiles that lie past the stored columns altogether, several to a pair (one pair walks all of them), either tile width
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("M,N,K,stored", [(512, 1024, 128, 64), (300, 640, 192, 8), (768, 1536, 64, 520)])
+def test_pair_gemm_stores_fewer_columns_than_it_computes(M, N, K, stored, residual):
+    from pmetal_b200.ops import native as nat
+    torch.manual_seed(N)
+    x, w, res = _rand(M, K), _rand(N, K, scale=K ** -0.5), _rand(M, N)
+    out = torch.full((M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    nat.raw_gemm(x, 0, K, M, w, 0, K, N, out, 0, N, M, N, K, R=res if residual else None, ldr=N if residual else 0, n_store=stored, bn=256,
+                 max_ctas=2)
+    ref = x.float() @ w.float().t()
+    _near(out[:, :stored], (ref + res.float() if residual else ref)[:, :stored], "stored columns")
+    assert bool((out[:, stored:] == 7).all())
+    nat.check_status()
