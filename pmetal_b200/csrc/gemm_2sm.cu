@@ -222,7 +222,7 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     // stores (whole 128-byte lines; a store from registers writes 16 bytes to each of 32 rows per instruction, which at
     // K = 1024 took longer than the tile's MMAs). A residual piece is brought into the same buffer by TMA beforehand.
     const int q = warp & 3;
-    const bool staged = p.out_mode == 0 && p.tail == nullptr;
+    const bool staged = p.staged;
     uint8_t* ebuf = epi + (warp - 2) * 8192;
     uint64_t* rb = r_bar + (warp - 2) * 2;
     const uint32_t row_off = static_cast<uint32_t>(lane) * 128u;
@@ -358,8 +358,10 @@ static int launch_pair(GemmParams p, const void* A, int lda, int a_rows, const v
     if ((rc = operand_map(&mb2, B2, p.b2_mn, b2_rows, p.K2, ldb2, T::kHalf))) return rc * 10 - 4;
   }
   md = mr = ma;
-  if (p.out_mode == 0 && !p.tail) {
-    // columns past n_store and rows past M lie outside the map: the store leaves them alone
+  // columns past n_store and rows past M lie outside the map and the store leaves them alone, but it cuts a row off at 16 bytes: where
+  // n_store ends inside 8 columns the results are stored from registers
+  p.staged = p.out_mode == 0 && !p.tail && p.n_store % 8 == 0;
+  if (p.staged) {
     if ((rc = make_map(&md, p.D, p.n_store, p.M, p.ldd, 64, 32))) return rc * 10 - 5;
     if (p.R && (rc = make_map(&mr, p.R, p.n_store, p.M, p.ldr, 64, 32))) return rc * 10 - 6;
   }

@@ -32,6 +32,7 @@ struct GemmParams {
   int seg_r;
   int tmem_cols;
   int group_m;     // CTA-pair kernel: row blocks per group of the tile order
+  int staged;      // CTA-pair kernel: results leave through shared memory as TMA stores
   int* status;
   float* ws;             // out_mode 6: [tiles][splits][128][bn] fp32 partial tiles
   unsigned* ws_cnt;      // out_mode 6: [tiles][4] arrival counters, zero between launches

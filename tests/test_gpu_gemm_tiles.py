@@ -47,7 +47,8 @@ def test_pair_gemm_tile_edges(M, N, K, segs):
 
 # tiles that lie past the stored columns altogether, several to a pair (one pair walks all of them), either tile width
 @pytest.mark.parametrize("residual", [False, True])
-@pytest.mark.parametrize("M,N,K,stored", [(512, 1024, 128, 64), (300, 640, 192, 8), (768, 1536, 64, 520)])
+@pytest.mark.parametrize("M,N,K,stored", [(512, 1024, 128, 64), (300, 640, 192, 8), (768, 1536, 64, 520),
+                                            (512, 1024, 128, 100), (768, 1536, 64, 513)])
 def test_pair_gemm_stores_fewer_columns_than_it_computes(M, N, K, stored, residual):
     from pmetal_b200.ops import native as nat
     torch.manual_seed(N)
@@ -58,4 +59,17 @@ def test_pair_gemm_stores_fewer_columns_than_it_computes(M, N, K, stored, residu
     ref = x.float() @ w.float().t()
     _near(out[:, :stored], (ref + res.float() if residual else ref)[:, :stored], "stored columns")
     assert bool((out[:, stored:] == 7).all())
+    nat.check_status()
+
+
+@pytest.mark.parametrize("N", [500, 251, 1023])
+def test_pair_gemm_into_a_wider_matrix(N):
+    """The last columns of the result end inside 16 bytes: what lies beside them in the same row stays."""
+    from pmetal_b200.ops import native as nat
+    torch.manual_seed(N)
+    x, w, wide = _rand(520, 256), _rand(N, 256, scale=1 / 16), _rand(520, 1032)
+    out = torch.full((520, 1032), 7.0, dtype=torch.bfloat16, device="cuda")
+    nat.gemm(x, w, residual=wide[:, :N], out=out[:, :N])
+    _near(out[:, :N], x.float() @ w.float().t() + wide[:, :N].float(), "result")
+    assert bool((out[:, N:] == 7).all())
     nat.check_status()
