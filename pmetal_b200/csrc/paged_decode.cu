@@ -12,9 +12,12 @@
 // int8: codes become bf16 exactly (|code| <= 127 has 7 bits); the scale of a (key, 64 channels) multiplies the partial score in
 // fp32, and the probability before its rounding to bf16, so a cached value is never rounded itself.
 //
-// Measured in a captured chain (here; 64-row tiles with one warp at work, or split keys and a merge kernel; bytes at 6.5 TB/s):
-//   64 x 450 keys, 16 heads on 8: 26.1, 33.0, 18.1 us      16 x 700: 13.6, 19.3, 7.1 us      1 x 6000: 11.2, 17.1, 3.8 us
-//   8 x 6000 keys: 38.6, 54.5, 30.2 us; int8: 44.3, 92.6, 16.1 us (expanding the codes)
+// Probabilities meet bf16 values as two bf16 (the rounded one and what it leaves, two products), about 2^-17 of each: one bf16 alone
+// costs 2 to 12 % of a sum whose terms nearly cancel. The second product takes 1 to 7 % of the kernel's time.
+//
+// Measured, captured over cold caches (here; 64-row tiles, split keys and a merge kernel; bytes at 6.5 TB/s):
+//   64 x 450 keys, 16 heads on 8: 29.3, 30.4, 18.1 us      16 x 700: 12.8, 15.7, 7.1 us      1 x 6000: 12.0, 18.0, 3.8 us
+//   8 x 6000 keys: 35.2, 42.0, 30.2 us; int8: 35.3, 69.3, 15.1 us (expanding the codes)
 #include <algorithm>
 
 #include "gemm_pair.cuh"
@@ -54,6 +57,10 @@ __device__ __forceinline__ float pd_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// what the two bf16 of `packed` leave of (a, b), as bf16
+__device__ __forceinline__ uint32_t pd_rest(float a, float b, uint32_t packed) {
+  return pack_bf16x2(a - __uint_as_float(packed << 16), b - __uint_as_float(packed & 0xffff0000u));
 }
 // byte i of a word of biased codes (code + 128) as the fp32 bits of the code: 2^23 + u has u in its low bits
 __device__ __forceinline__ uint32_t pd_code(uint32_t biased, int i) {
@@ -292,7 +299,9 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         }
       }
     } else {
+      // probabilities keep 16 bits of their mantissa: the bf16 value and, in a second product, what it leaves
       const uint32_t pb0 = pack_bf16x2(pr[0][0], pr[0][1]), pb1 = pack_bf16x2(pr[1][0], pr[1][1]);
+      const uint32_t pl0 = pd_rest(pr[0][0], pr[0][1], pb0), pl1 = pd_rest(pr[1][0], pr[1][1], pb1);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         uint4 vr[4];
@@ -303,8 +312,10 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
           uint32_t x[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u) x[u] = w == 0 ? vr[u].x : w == 1 ? vr[u].y : w == 2 ? vr[u].z : vr[u].w;
-          pd_mma(o[h * 4 + w], __byte_perm(x[0], x[1], 0x5410), __byte_perm(x[0], x[1], 0x7632), __byte_perm(x[2], x[3], 0x5410),
-                 __byte_perm(x[2], x[3], 0x7632), pb0, pb1);
+          const uint32_t a0 = __byte_perm(x[0], x[1], 0x5410), a1 = __byte_perm(x[0], x[1], 0x7632), a2 = __byte_perm(x[2], x[3], 0x5410),
+                         a3 = __byte_perm(x[2], x[3], 0x7632);
+          pd_mma(o[h * 4 + w], a0, a1, a2, a3, pb0, pb1);
+          pd_mma(o[h * 4 + w], a0, a1, a2, a3, pl0, pl1);
         }
       }
     }

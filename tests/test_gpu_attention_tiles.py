@@ -97,6 +97,35 @@ def test_paged_decode_attention(quant, hq, hkv, lens, qlens, splits):
         at += m
 
 
+@pytest.mark.parametrize("hq,hkv", [(2, 2), (4, 2), (8, 1)])
+@pytest.mark.parametrize("n,splits", [(64, 1), (333, 2), (2100, 8)])
+def test_paged_decode_keeps_its_probabilities(hq, hkv, n, splits):
+    """Values of opposite sign at keys that nearly agree: what is left of the sum is about 2 % of a probability, where a probability
+    rounded to bf16 (2^-9) would leave errors of several per cent of it."""
+    from pmetal_b200.models.kv_cache import PagedKVCache
+    from pmetal_b200.ops import native as nat
+    g = torch.Generator(device="cuda").manual_seed(n + hq)
+    cache = PagedKVCache(1, hkv, 128, 48)
+    cache.add_sequence(0)
+    if n > 1:
+        cache.reserve(0, n - 1)
+    meta = cache.prepare([0], [1])
+    k, v = (torch.randn(48 * 64, hkv, 128, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    k[1::2] = (k[::2].float() + 0.02 * torch.randn(k[::2].shape, device="cuda", generator=g)).to(torch.bfloat16)
+    v[1::2] = -v[::2]
+    cache.write_reference(0, k, v, torch.arange(48 * 64, device="cuda"))
+    q = torch.randn(1, hq, 128, device="cuda", generator=g).to(torch.bfloat16)
+    out, p = torch.empty_like(q), nat._p
+    assert nat.lib().pm_paged_decode(p(q), p(cache.k[0]), p(cache.v[0]), p(None), p(None), p(out), p(meta.block_table), p(meta.seq_lens),
+                                     p(meta.q_start), p(meta.q_lens), nat.c_int(1), nat.c_int(meta.block_table.shape[1]), nat.c_int(48),
+                                     nat.c_int(1), nat.c_int(hq), nat.c_int(hkv), nat.c_float(128 ** -0.5), nat.c_int(splits),
+                                     p(nat.status_word(q.device)), nat._stream()) == 0
+    kk, vv = (t.double().repeat_interleave(hq // hkv, 1) for t in cache.gather(0, 0))
+    s = torch.einsum("hd,jhd->hj", q[0].double(), kk) * 128 ** -0.5
+    want = torch.einsum("hj,jhd->hd", s.softmax(-1), vv)
+    assert float((out[0].double() - want).norm() / want.norm()) < 4e-3       # one bf16 rounding of the output
+
+
 def test_paged_dispatch_keeps_small_steps_on_the_split_kernel():
     from pmetal_b200.ops.native import _paged_on_tensor_cores as tc
     assert tc(1, 2048, 2048, 16, 8) and tc(6, 700, 700, 16, 8) and tc(1, 512, 12000, 16, 8)
