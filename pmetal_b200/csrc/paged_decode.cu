@@ -12,12 +12,15 @@
 // int8: codes become bf16 exactly (|code| <= 127 has 7 bits); the scale of a (key, 64 channels) multiplies the partial score in
 // fp32, and the probability before its rounding to bf16, so a cached value is never rounded itself.
 //
+// The last block may hold anything past the keys, what a sequence that gave the block back left there included (NaN, infinities): scores
+// there are replaced, values are taken as zero, since a probability of zero would not silence them.
+//
 // Probabilities meet bf16 values as two bf16 (the rounded one and what it leaves, two products), about 2^-17 of each: one bf16 alone
-// costs 2 to 12 % of a sum whose terms nearly cancel. The second product takes 1 to 7 % of the kernel's time.
+// costs 2 to 12 % of a sum whose terms nearly cancel. The second product takes up to 3 % of the kernel's time.
 //
 // Measured, captured over cold caches (here; 64-row tiles, split keys and a merge kernel; bytes at 6.5 TB/s):
-//   64 x 450 keys, 16 heads on 8: 29.3, 30.4, 18.1 us      16 x 700: 12.8, 15.7, 7.1 us      1 x 6000: 12.0, 18.0, 3.8 us
-//   8 x 6000 keys: 35.2, 42.0, 30.2 us; int8: 35.3, 69.3, 15.1 us (expanding the codes)
+//   64 x 450 keys, 16 heads on 8: 28.9, 30.4, 18.1 us      16 x 700: 12.5, 15.7, 7.1 us      1 x 6000: 11.5, 18.0, 3.8 us
+//   8 x 6000 keys: 34.5, 42.0, 30.2 us; int8: 35.5, 69.3, 15.1 us (expanding the codes)
 #include <algorithm>
 
 #include "gemm_pair.cuh"
@@ -219,7 +222,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         const int key = 2 * t4 + (u & 1) + (u >> 1) * 8;
         const float2* sc = reinterpret_cast<const float2*>(smem + st * kStage + 2 * kPdBox) + quarter + key;
         ks[u >> 1][u & 1] = sc[0];
-        vs[u] = sc[64];
+        vs[u] = j0 + key < kv ? sc[64] : make_float2(0.f, 0.f);
       }
     }
     float s[2][2];
@@ -306,7 +309,11 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       for (int h = 0; h < 2; ++h) {
         uint4 vr[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) vr[u] = pd_lds16(vbox + h * kPdBox, quarter + 2 * t4 + (u & 1) + (u >> 1) * 8, g);
+        for (int u = 0; u < 4; ++u) {
+          const int key = 2 * t4 + (u & 1) + (u >> 1) * 8;
+          vr[u] = pd_lds16(vbox + h * kPdBox, quarter + key, g);
+          if (j0 + key >= kv) vr[u] = make_uint4(0u, 0u, 0u, 0u);
+        }
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
           uint32_t x[4];

@@ -56,6 +56,19 @@ def test_paged_prompt_attention(hq, hkv, lens, qlens):
     nat.check_status()
 
 
+def _paged_decode(q, cache, meta, splits=0):
+    from pmetal_b200.ops import native as nat
+    p, c = nat._p, nat.c_int
+    out = torch.full_like(q, float("nan"))
+    scales = (cache.k_scale[0], cache.v_scale[0]) if cache.quant else (None, None)
+    rc = nat.lib().pm_paged_decode(p(q), p(cache.k[0]), p(cache.v[0]), p(scales[0]), p(scales[1]), p(out), p(meta.block_table),
+                                   p(meta.seq_lens), p(meta.q_start), p(meta.q_lens), c(meta.block_table.shape[0]),
+                                   c(meta.block_table.shape[1]), c(cache.num_blocks), c(meta.max_q), c(q.shape[1]), c(cache.hkv),
+                                   nat.c_float(128 ** -0.5), c(splits), p(nat.status_word(q.device)), nat._stream())
+    assert rc == 0
+    return out
+
+
 # (kv lengths, new tokens): ends on and beside the 16-key quarters and the 64-key blocks, fewer blocks than slices, several tokens
 DECODE = [([1, 15, 16, 17], [1, 1, 1, 1]), ([63, 64, 65, 700], [1, 1, 1, 1]), ([130, 5], [5, 2]), ([2100], [8])]
 
@@ -103,7 +116,6 @@ def test_paged_decode_keeps_its_probabilities(hq, hkv, n, splits):
     """Values of opposite sign at keys that nearly agree: what is left of the sum is about 2 % of a probability, where a probability
     rounded to bf16 (2^-9) would leave errors of several per cent of it."""
     from pmetal_b200.models.kv_cache import PagedKVCache
-    from pmetal_b200.ops import native as nat
     g = torch.Generator(device="cuda").manual_seed(n + hq)
     cache = PagedKVCache(1, hkv, 128, 48)
     cache.add_sequence(0)
@@ -115,15 +127,38 @@ def test_paged_decode_keeps_its_probabilities(hq, hkv, n, splits):
     v[1::2] = -v[::2]
     cache.write_reference(0, k, v, torch.arange(48 * 64, device="cuda"))
     q = torch.randn(1, hq, 128, device="cuda", generator=g).to(torch.bfloat16)
-    out, p = torch.empty_like(q), nat._p
-    assert nat.lib().pm_paged_decode(p(q), p(cache.k[0]), p(cache.v[0]), p(None), p(None), p(out), p(meta.block_table), p(meta.seq_lens),
-                                     p(meta.q_start), p(meta.q_lens), nat.c_int(1), nat.c_int(meta.block_table.shape[1]), nat.c_int(48),
-                                     nat.c_int(1), nat.c_int(hq), nat.c_int(hkv), nat.c_float(128 ** -0.5), nat.c_int(splits),
-                                     p(nat.status_word(q.device)), nat._stream()) == 0
+    out = _paged_decode(q, cache, meta, splits)
     kk, vv = (t.double().repeat_interleave(hq // hkv, 1) for t in cache.gather(0, 0))
     s = torch.einsum("hd,jhd->hj", q[0].double(), kk) * 128 ** -0.5
     want = torch.einsum("hj,jhd->hd", s.softmax(-1), vv)
     assert float((out[0].double() - want).norm() / want.norm()) < 4e-3       # one bf16 rounding of the output
+
+
+@pytest.mark.parametrize("quant", [None, "int8"])
+@pytest.mark.parametrize("left", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("lens,qlens", [([1, 15, 33, 64, 190], [1, 1, 1, 1, 1]), ([70, 9], [5, 8])])
+def test_paged_decode_ignores_what_lies_past_the_keys(quant, left, lens, qlens):
+    """A block that another sequence has given back keeps its contents: they do not reach the sequence that has it now."""
+    from pmetal_b200.models.kv_cache import PagedKVCache
+    g = torch.Generator(device="cuda").manual_seed(len(lens))
+    cache = PagedKVCache(1, 2, 128, 16, quant=quant)
+    for i, (n, m) in enumerate(zip(lens, qlens)):
+        cache.add_sequence(i)
+        if n > m:
+            cache.reserve(i, n - m)
+    meta = cache.prepare(list(range(len(lens))), qlens)
+    every = torch.arange(16 * 64, device="cuda")
+    k, v = (torch.randn(16 * 64, 2, 128, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    cache.write_reference(0, k, v, every)
+    q = torch.randn(sum(qlens), 4, 128, device="cuda", generator=g).to(torch.bfloat16)
+    clean = _paged_decode(q, cache, meta)
+    held = torch.cat([torch.tensor(cache.seqs[i].blocks)[torch.arange(n) // 64] * 64 + torch.arange(n) % 64 for i, n in enumerate(lens)])
+    other = torch.ones(16 * 64, dtype=torch.bool)
+    other[held] = False
+    for t in ((cache.k_scale[0], cache.v_scale[0]) if quant else (cache.k[0], cache.v[0])):
+        t.view(16 * 64, -1)[other.cuda()] = left
+    got = _paged_decode(q, cache, meta)
+    assert bool(torch.isfinite(clean).all()) and bool((got == clean).all())
 
 
 def test_paged_dispatch_keeps_small_steps_on_the_split_kernel():
