@@ -327,19 +327,20 @@ def lora_t(x, a, scale: float) -> torch.Tensor:
 
 
 def lora_dt(dy, b, seg_sizes, r, scale) -> torch.Tensor:
-    """dt[:, seg*r:(seg+1)*r] = scale * dy[:, seg] b_seg   ([M, 64-padded]); padding columns are unspecified."""
+    """dt[:, seg*r:(seg+1)*r] = scale * dy[:, seg] b_seg   ([M, 64-padded]; padding columns are zero: the product with A reads 16 at a time)."""
     M, N = dy.shape
     nseg = len(seg_sizes)
     if MN_MAJOR and nseg * r <= 64 and nseg <= 4 and all(s % 64 == 0 for s in seg_sizes) and b.shape[1] == r:
         dt = _lora_tall(dy, b, 1, r, seg_sizes, scale)
         if dt is not None:
             return dt
-    dt = torch.empty(M, _t_width(nseg * r), dtype=torch.bfloat16, device=dy.device)
+    dt = torch.zeros(M, _t_width(nseg * r), dtype=torch.bfloat16, device=dy.device)
     b_t = b.t().contiguous()                      # [r, N], K-major over N
+    bn = 32 if r <= 32 else 64
     n0 = 0
     for i, sz in enumerate(seg_sizes):
-        raw_gemm(dy[:, n0:], 0, dy.stride(0), M, b_t[:, n0:], 0, N, r, dt[:, i * r:], 0, dt.stride(0), M, 32, sz,
-                 n_store=r, alpha=scale, bn=32)
+        raw_gemm(dy[:, n0:], 0, dy.stride(0), M, b_t[:, n0:], 0, N, r, dt[:, i * r:], 0, dt.stride(0), M,
+                 -(-r // bn) * bn, sz, n_store=r, alpha=scale, bn=bn)
         n0 += sz
     return dt
 
@@ -529,6 +530,8 @@ def lora_db(dy, t, seg_sizes, r: int, out: torch.Tensor) -> None:
         return
     nk = -(-M // 64)
     det = DETERMINISTIC
+    wide = _t_width(r)                             # tiles of 64 columns that cover the rank
+    n_wide = wide // 64
     if any(s % 128 for s in seg_sizes[:-1]):       # a 128-row tile of the launch below would straddle two segments
         n0 = 0
         for i, sz in enumerate(seg_sizes):
@@ -536,12 +539,12 @@ def lora_db(dy, t, seg_sizes, r: int, out: torch.Tensor) -> None:
             if (d.data_ptr() | ti.data_ptr()) % 16:
                 o.add_(d.t().float() @ ti[:, :r].float())
             else:
-                raw_gemm(d, 1, dy.stride(0), sz, ti, 1, t.stride(0), t.shape[1] - i * r, o, 4 if det else 2, out.stride(0), sz, 64, M,
-                         n_store=r, bn=64, splits=1 if det else _splits_for(-(-sz // 128), nk))
+                raw_gemm(d, 1, dy.stride(0), sz, ti, 1, t.stride(0), t.shape[1] - i * r, o, 4 if det else 2, out.stride(0), sz, wide,
+                         M, n_store=r, bn=64, splits=1 if det else _splits_for(-(-sz // 128) * n_wide, nk))
             n0 += sz
         return
-    raw_gemm(dy, 1, dy.stride(0), N, t, 1, t.stride(0), t.shape[1], out, 4 if det else 2, out.stride(0), N, 64, M,
-             n_store=r, bn=64, splits=1 if det else _splits_for(-(-N // 128), nk),
+    raw_gemm(dy, 1, dy.stride(0), N, t, 1, t.stride(0), t.shape[1], out, 4 if det else 2, out.stride(0), N, wide, M,
+             n_store=r, bn=64, splits=1 if det else _splits_for(-(-N // 128) * n_wide, nk),
              seg_mode=2 if len(seg_sizes) > 1 else 0, seg_sizes=seg_sizes, seg_r=r)
 
 

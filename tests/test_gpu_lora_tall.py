@@ -71,3 +71,30 @@ def test_lora_layer_in_one_call(M, segs, r, K, transposed):
     assert _rel(y.detach(), want.detach()) < 4e-3                    # bf16 t and y
     for p, q in zip(got, torch.autograd.grad(want, (xr, ar, br), dy.float())):
         assert _rel(p, q) < 6e-3                                     # bf16 dt, t and dx
+
+
+# ranks whose segments are wider than one tile of the general path, together or each; padding columns beside a multiple of 8
+@pytest.mark.parametrize("segs,r", [((128, 64), 64), ((256, 128, 128), 64), ((256,), 128), ((128, 128), 96), ((128, 64, 64), 24), ((96, 32), 64),
+                                    ((192,), 72)])
+@pytest.mark.parametrize("M", [100, 300])
+def test_gradients_of_wide_ranks(segs, r, M):
+    from pmetal_b200.ops import functional as ops
+    g = torch.Generator(device="cuda").manual_seed(M + r)
+    K, N, nr = 136, sum(segs), r * len(segs)
+    f = lambda *s: torch.randn(*s, device="cuda", generator=g)      # noqa: E731
+    x, dy = f(M, K).to(torch.bfloat16).requires_grad_(True), f(M, N).to(torch.bfloat16)
+    w = (f(N, K) * K ** -0.5).to(torch.bfloat16)
+    a, b = (f(nr, K) * K ** -0.5).requires_grad_(True), (f(N, r) * 0.1).requires_grad_(True)
+    y = ops.lora_linear(x, w, None, a, b, segs, r, 2.0)
+    poison = [torch.full((n,), float("nan"), dtype=torch.bfloat16, device="cuda") for n in (M * 64, M * 128, M * 192, M * 256) for _ in range(8)]
+    del poison                                             # what the products allocate next holds NaN where they do not write
+    got = torch.autograd.grad(y, (x, a, b), dy)
+    xr, ar, br = (t.detach().to(torch.bfloat16).float().requires_grad_(True) for t in (x, a, b))
+    parts, at = [], 0
+    for i, n in enumerate(segs):
+        parts.append(2.0 * (xr @ ar[i * r:(i + 1) * r].t()) @ br[at:at + n].t())
+        at += n
+    want = xr @ w.float().t() + torch.cat(parts, -1)
+    assert _rel(y.detach(), want.detach()) < 4e-3                    # bf16 t and y
+    for name, p, q in zip(("x", "a", "b"), got, torch.autograd.grad(want, (xr, ar, br), dy.float())):
+        assert _rel(p, q) < 6e-3, name                               # bf16 dt, t and dx
