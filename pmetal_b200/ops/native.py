@@ -1004,12 +1004,36 @@ def _paged_splits(n_seq: int, max_kv: int, hkv: int) -> int:
     return max(1, min(n_blocks // 4, 2 * sm_count() // max(ctas, 1), 32)) if ctas < sm_count() else 1
 
 
+def _paged_tokens_apart(n_seq: int, max_q: int, max_kv: int, hkv: int, table: int, int8: bool) -> bool:
+    """Whether a step of 2 to 8 tokens per sequence is faster on the decode kernel, which streams the keys once per token, than on the
+    64-row kernel, which streams them once for all of them. Estimates in us that fit the measured times: the first takes its rounds of CTAs
+    times the key blocks that one CTA walks, the second mostly its key blocks. Measured (decode kernel, 64-row kernel), 16 heads on 8:
+    1 x 500 keys, 5 tokens 6.0, 10.2; 1 x 6000, 3 tokens 13.7, 17.8, 5 tokens 21.2, 17.0; 4 x 1500, 2 tokens 10.4, 13.5, 5 tokens 20.4, 14.0;
+    16 x 700, 2 tokens 13.7, 15.7, 4 tokens 24.8, 15.8; 64 x 450, 2 tokens 32.6, 30.8, 8 tokens 86.1, 31.9; 8 x 6000, 2 tokens 45.4, 42.3;
+    int8: 2 tokens 59.7, 69.4, 3 tokens 109.5, 69.5."""
+    sms, blocks = sm_count(), -(-max_kv // 64)
+    ctas, splits = n_seq * max_q * hkv, 1
+    while splits < 8 and ctas * splits * 2 <= 2 * sms and splits * 2 <= max(table, 8):      # as pm_paged_decode does
+        splits *= 2
+    ctas *= splits
+    per_sm = min(-(-ctas // sms), 2 if int8 else 3)
+    rounds = -(-ctas // (sms * per_sm))
+    if not int8 and splits == 8 and sms * 4 // 5 < ctas <= sms:      # 15 clusters of 8 fit at one CTA per SM
+        rounds = 2
+    walk = rounds * -(-blocks // splits)
+    apart = 5 + walk * (0.76 if per_sm == 1 else 1.16) if int8 else 4.5 + walk * (0.63, 0.92, 1.2)[per_sm - 1]
+    keys = n_seq * hkv * blocks
+    together = (11 + 0.0085 * keys if int8 else 9 + 0.0052 * keys) + 0.2 * _paged_splits(n_seq, max_kv, hkv)
+    return apart <= together + 1.5          # in a chain of dependent launches the first starts under its predecessor's tail
+
+
 def _paged_route(meta, hq: int, hkv: int, int8: bool):
-    """(kernel, slices of the keys) for attention over a bf16 or int8 paged cache without a window: steps of up to 8 tokens per sequence
-    and 8 heads per group stream the keys once per token (csrc/paged_decode.cu), prompts fill tensor-core tiles where
-    ``_paged_on_tensor_cores`` says so, the rest goes to the 64-row kernel."""
+    """(kernel, slices of the keys) for attention over a bf16 or int8 paged cache without a window: single tokens, and a few per sequence
+    where ``_paged_tokens_apart`` says so, stream the keys once per token (csrc/paged_decode.cu, up to 8 heads per group), prompts fill
+    tensor-core tiles where ``_paged_on_tensor_cores`` says so, the rest goes to the 64-row kernel."""
     n_seq = meta.block_table.shape[0]
-    if meta.max_q <= 8 and hq // hkv <= 8:
+    if hq // hkv <= 8 and (meta.max_q == 1 or (meta.max_q <= 8 and _paged_tokens_apart(n_seq, meta.max_q, meta.max_kv, hkv,
+                                                                                      meta.block_table.shape[1], int8))):
         return PAGED_DECODE, 1
     if not int8 and _paged_on_tensor_cores(n_seq, meta.max_q, meta.max_kv, hq, hkv):
         return PAGED_TENSOR, 1

@@ -135,3 +135,17 @@ def test_stream_gradient_of_one_half_passes_nothing_for_the_other(monkeypatch, r
     h_out, dh_in, dx_out, h_pre, h_post, h_res = (a.value for a in calls[0][1:7])
     assert (dh_in is not None) == (h_pre is not None) == read_half
     assert (dx_out is None) == (h_out is None) == (h_post is None) == (h_res is None) == read_half
+
+
+# (int8, sequences, keys, tokens per sequence, heads, kv heads, whether the decode kernel measured clearly faster than the 64-row kernel)
+@pytest.mark.parametrize("int8,n,ctx,q,hq,hkv,apart", [
+    (0, 1, 500, 8, 16, 8, True), (0, 1, 6000, 3, 16, 8, True), (0, 1, 6000, 2, 16, 8, False), (0, 1, 6000, 8, 16, 8, False), (0, 4, 1500, 2, 16, 8, True),
+    (0, 4, 1500, 5, 16, 8, False), (0, 16, 700, 2, 16, 8, True), (0, 16, 700, 4, 16, 8, False), (0, 64, 450, 2, 16, 8, False), (0, 64, 450, 8, 16, 8, False),
+    (0, 8, 6000, 2, 16, 8, False), (0, 8, 6000, 8, 32, 4, False), (0, 64, 450, 1, 16, 8, True), (0, 64, 450, 1, 64, 4, False),
+    (1, 1, 6000, 4, 16, 8, True), (1, 1, 6000, 5, 16, 8, False), (1, 64, 450, 2, 16, 8, True), (1, 64, 450, 3, 16, 8, False), (1, 8, 6000, 2, 16, 8, True),
+    (1, 8, 6000, 3, 16, 8, False), (1, 8, 6000, 1, 16, 8, True)])
+def test_steps_of_a_few_tokens_take_the_faster_attention_kernel(int8, n, ctx, q, hq, hkv, apart):
+    from pmetal_b200.models.kv_cache import BatchMeta
+    from pmetal_b200.ops import native
+    meta = BatchMeta(list(range(n)), torch.zeros(n, ctx // 64 + 1, dtype=torch.int32), None, None, None, None, None, n * q, q, ctx)
+    assert (native._paged_route(meta, hq, hkv, bool(int8))[0] == native.PAGED_DECODE) == apart
