@@ -253,8 +253,9 @@ __device__ __forceinline__ void merge_slices(const float* part, int ctas, float&
 
 // What bounds it: a row is 300 KB, which one CTA walked in 60 us for the greedy answer, two bytes per load, and nine times more
 // for top-k and top-p. The CTAs of a row's cluster take a slice each of every pass, with 16-byte loads, and merge through
-// distributed shared memory; maximum, index and partition function come out of one pass. 151936 bf16 logits, launched one by one, start and
-// now: greedy 1 row 64, 15 us, 64 rows 64, 15 us (15 us is what launching costs); top-k 20 and top-p 0.8: 1458, 223 us and 1461, 436 us.
+// distributed shared memory; maximum, index and partition function come out of one pass. 151936 bf16 logits, launched one by one, with one
+// CTA to a row and with a cluster: greedy 1 row 64, 15 us, 64 rows 64, 15 us (15 us is what launching costs); top-k 20 and top-p 0.8:
+// 1458, 223 us and 1461, 436 us. A row in which nothing can be chosen (-inf or NaN throughout) gives token 0 and log-probability NaN.
 __global__ void __launch_bounds__(kSampThreads) sample_kernel(const SampleParams p) {
   __shared__ float hist[2][256], total[256];
   __shared__ float red[64];
@@ -314,8 +315,8 @@ __global__ void __launch_bounds__(kSampThreads) sample_kernel(const SampleParams
   const float m = mv;
   if (greedy) {
     if (rank == 0 && threadIdx.x == 0) {
-      p.out_token[r] = mi;
-      if (p.out_logprob) p.out_logprob[r] = -__logf(z);
+      p.out_token[r] = mi < p.vocab ? mi : 0;         // a row without a value above -inf
+      if (p.out_logprob) p.out_logprob[r] = mi < p.vocab ? -__logf(z) : NAN;
     }
     leave();
     return;
@@ -373,8 +374,8 @@ __global__ void __launch_bounds__(kSampThreads) sample_kernel(const SampleParams
     }
   }
   if (rank == 0 && threadIdx.x == 0) {
-    p.out_token[r] = bi;
-    if (p.out_logprob) p.out_logprob[r] = (row.at(bi) - m) * inv_t - __logf(zt);
+    p.out_token[r] = bi < p.vocab ? bi : 0;           // nothing survived: a row of -inf or NaN
+    if (p.out_logprob) p.out_logprob[r] = bi < p.vocab ? (row.at(bi) - m) * inv_t - __logf(zt) : NAN;
   }
   leave();
 }

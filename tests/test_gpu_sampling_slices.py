@@ -41,3 +41,18 @@ def test_drawn_tokens_survive_the_filters(V, kw):
         q = torch.log_softmax(keep / 0.8, -1).gather(1, ids[:, None])[:, 0]
         ok = q > float("-inf")
         assert float((lp - q)[ok].abs().max()) < 0.05      # a tied token more or less in the nucleus
+
+
+@pytest.mark.parametrize("V", [37, 16391, 151936])
+@pytest.mark.parametrize("kw", [dict(temperature=0.0), dict(temperature=0.8, do_sample=True, top_k=5), dict(temperature=1.0, do_sample=True, top_p=0.5)])
+@pytest.mark.parametrize("bad", [float("-inf"), float("nan")])
+def test_rows_without_a_choice(V, kw, bad):
+    """A row in which every logit is -inf or NaN gives a token of the vocabulary; its neighbours are what they are alone."""
+    from pmetal_b200.models.sampling import Sampler, SamplingParams
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randn(3, V, device="cuda", generator=g)
+    x[1] = bad
+    x[2, 1:] = float("-inf")
+    ids, lp = Sampler(SamplingParams(seed=3, **kw), "cuda").sample(x, return_logprobs=True)
+    assert int(ids[1]) == 0 and bool(torch.isnan(lp[1])) and int(ids[2]) == 0 and abs(float(lp[2])) < 1e-5
+    assert 0 <= int(ids[0]) < V and bool(torch.isfinite(lp[0]))
