@@ -525,7 +525,8 @@ class DecoderLM(nn.Module):
             for lin in (at._modules["qkv_proj"], at._modules["o_proj"], mlp._modules["gate_up_proj"], mlp._modules["down_proj"]):
                 p, own = lin._parameters["weight"], lin.__dict__
                 if (lin._parameters.get("bias") is not None or lin._parameters.get("lora_a") is not None or own.get("lora_a") is not None
-                        or own.get("qweight") is not None or own.get("batched") is not None or p.requires_grad or p.dtype != dt
+                        or own.get("qweight") is not None or (own.get("batched") is not None and own.get("adapter_rows") is not None)
+                        or p.requires_grad or p.dtype != dt
                         or p.dim() != 2 or not p.is_contiguous() or p.data_ptr() % 16):
                     return None
                 w.append(p.data_ptr())

@@ -105,3 +105,20 @@ def test_generation_with_per_request_adapters_matches_single_adapter_models(tmp_
         eng.submit(Request([1, 2], SamplingParams.greedy(2), adapter="gamma"))
     ads.unload("beta")
     assert ads.names[1] is None and ads.load("beta2", d2) == 1
+
+
+def test_adapters_that_are_off_leave_the_one_call_forward_open():
+    from pmetal_b200.models.config import ModelArgs
+    from pmetal_b200.models.decoder import DecoderLM
+    m = DecoderLM(ModelArgs(vocab_size=64, hidden_size=128, intermediate_size=128, num_hidden_layers=2, num_attention_heads=2,
+                            num_key_value_heads=1, head_dim=128), torch.bfloat16)
+    for p in m.parameters():
+        p.requires_grad_(False)
+    cache = m.new_cache(4)
+    plain = m._stack_addresses(cache)
+    ads = AdapterSet(m, 2, 4)
+    assert plain is not None and m._stack_addresses(cache) == plain
+    ads.set_rows([0, NO_ADAPTER])
+    assert m._stack_addresses(cache) is None
+    ads.set_rows(None)
+    assert m._stack_addresses(cache) == plain
