@@ -21,6 +21,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from ..ops import functional as ops
 from .config import ModelArgs
@@ -32,6 +33,11 @@ ALL_PROJ = ATTN_PROJ + MLP_PROJ
 
 # rows up to which linear layers run on the bandwidth-bound mat-vec kernel instead of tensor-core tiles (decode)
 GEMV_MAX_ROWS = int(os.environ.get("PMETAL_GEMV_MAX_ROWS", "16"))
+
+
+def _call_is_wrapped(own: Dict) -> bool:
+    """Whether calling the module with this ``__dict__`` runs more than its class's ``forward``."""
+    return bool(own["_forward_hooks"] or own["_forward_pre_hooks"]) or "forward" in own
 
 
 class FusedLinear(nn.Module):
@@ -508,26 +514,30 @@ class DecoderLM(nn.Module):
 
     def _stack_addresses(self, cache) -> Optional[List[int]]:
         """Device addresses of every layer in the order of ``pm_layer_stack``, or None where a layer is not a dense one with plain
-        bf16 weights (adapters, packed weights, biases, experts, sliding windows, sharding) or the cache is not a bf16 or int8 one.
+        bf16 weights (adapters, packed weights, biases, experts, sliding windows, sharding), where calling a module does more than its
+        weights say (hooks, a ``forward`` of the instance, parametrisations), or where the cache is not a bf16 or int8 one.
         Looked up on every call: adapters and packed weights come and go."""
         cfg = self.cfg
         if (cfg.attn_logit_softcap > 0 or getattr(self, "tp_world", 1) > 1 or cache.quant not in (None, "int8") or cache.window > 0
-                or cfg.hidden_size % 8 or cfg.intermediate_size % 8 or (cache.quant is None and cache.k[0].dtype != torch.bfloat16)):
+                or cfg.hidden_size % 8 or cfg.intermediate_size % 8 or (cache.quant is None and cache.k[0].dtype != torch.bfloat16)
+                or _has_any_global_hook()):
             return None
         rows: List[int] = []
         dt = torch.bfloat16
         for li, layer in enumerate(self.layers):
             mods = layer._modules
             at, mlp = mods["self_attn"], mods["mlp"]
-            if at.window or not isinstance(mlp, MLP):
+            if at.window or type(mlp) is not MLP or _call_is_wrapped(mlp.__dict__):
                 return None
             w = []
             for lin in (at._modules["qkv_proj"], at._modules["o_proj"], mlp._modules["gate_up_proj"], mlp._modules["down_proj"]):
-                p, own = lin._parameters["weight"], lin.__dict__
-                if (lin._parameters.get("bias") is not None or lin._parameters.get("lora_a") is not None or own.get("lora_a") is not None
-                        or own.get("qweight") is not None or (own.get("batched") is not None and own.get("adapter_rows") is not None)
-                        or p.requires_grad or p.dtype != dt
-                        or p.dim() != 2 or not p.is_contiguous() or p.data_ptr() % 16):
+                own = lin.__dict__
+                par = own["_parameters"]
+                p = par.get("weight")
+                if (p is None or type(lin) is not FusedLinear or _call_is_wrapped(own) or par.get("bias") is not None
+                        or par.get("lora_a") is not None or own.get("lora_a") is not None or own.get("qweight") is not None
+                        or (own.get("batched") is not None and own.get("adapter_rows") is not None)
+                        or p.requires_grad or p.dtype != dt or p.dim() != 2 or not p.is_contiguous() or p.data_ptr() % 16):
                     return None
                 w.append(p.data_ptr())
             norms = layer._parameters["input_layernorm"], layer._parameters["post_attention_layernorm"]

@@ -201,3 +201,40 @@ def test_rotated_4bit_cache_reference_path():
     assert rel < 0.12, rel                          # 4-bit Lloyd-Max on unit-variance coordinates: about 10 % error
     with pytest.raises(ValueError):
         model.new_cache(8, quant="q2")
+
+
+def _stackable():
+    from pmetal_b200.models.config import ModelArgs
+    m = DecoderLM(ModelArgs(vocab_size=64, hidden_size=128, intermediate_size=128, num_hidden_layers=2, num_attention_heads=2,
+                            num_key_value_heads=1, head_dim=128), torch.bfloat16)
+    for p in m.parameters():
+        p.requires_grad_(False)
+    return m, m.new_cache(4)
+
+
+@pytest.mark.parametrize("where", ["self_attn.qkv_proj", "self_attn.o_proj", "mlp", "mlp.gate_up_proj", "mlp.down_proj"])
+def test_wrapped_modules_keep_the_layer_by_layer_forward(where):
+    """Hooks, a forward of the instance, another class: what the module's call adds is not in its weights, so the one-call forward, which
+    reads only those, is not taken."""
+    from torch.nn.utils import parametrize
+    m, cache = _stackable()
+    mod = m.layers[1].get_submodule(where)
+    plain = m._stack_addresses(cache)
+    assert plain is not None
+    for register in (mod.register_forward_hook, mod.register_forward_pre_hook):
+        hook = register(lambda *a: None)
+        assert m._stack_addresses(cache) is None
+        hook.remove()
+        assert m._stack_addresses(cache) == plain
+    mod.forward = lambda x, residual=None: x
+    assert m._stack_addresses(cache) is None
+    del mod.forward
+    hook = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    assert m._stack_addresses(cache) is None
+    hook.remove()
+    mod.__class__ = type("Other", (type(mod),), {})
+    assert m._stack_addresses(cache) is None
+    if where != "mlp":
+        m, cache = _stackable()
+        parametrize.register_parametrization(m.layers[1].get_submodule(where), "weight", torch.nn.Identity())
+        assert m._stack_addresses(cache) is None
