@@ -411,10 +411,12 @@ class DecoderLM(nn.Module):
         T = x.shape[0]
         skinny = native and T <= GEMV_MAX_ROWS
         layers = self.layers
-        addresses = self._stack_addresses(cache) if native else None
+        addresses = None
+        if native:
+            from ..ops import native as nat
+            addresses = self._stack_addresses(cache) if nat.layer_stack_ok(T) else None
         if addresses is not None:
             # dense layers without adapters: all of them in one call of the runtime (csrc/layer_stack.cu)
-            from ..ops import native as nat
             x = nat.layer_stack(addresses, x.contiguous(), meta, rope[0], rope[1], hq, hkv, cfg.intermediate_size, cache.num_blocks,
                                 cfg.rms_norm_eps, d ** -0.5)
             layers = ()

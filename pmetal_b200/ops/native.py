@@ -24,7 +24,9 @@ LIB_PATH = os.environ.get("PMETAL_NATIVE_LIB") or os.path.join(
 MN_MAJOR = os.environ.get("PMETAL_MN_MAJOR", "1") == "1"
 ATTN_TC = os.environ.get("PMETAL_ATTN_TC", "1") == "1"      # tcgen05 attention kernels
 ATTN_FWD_V1 = os.environ.get("PMETAL_ATTN_FWD_V1", "0") == "1"   # single-softmax-group forward (comparison runs)
-USE_2SM = os.environ.get("PMETAL_GEMM_2SM", "1") == "1"   # CTA-pair kernel for 256-wide tiles
+# CTA-pair GEMM kernel for wide tiles on at least 256 rows. With PMETAL_GEMM_2SM=0 every GEMM runs on single CTAs, and the entries that issue
+# several launches from C++ (csrc/lora_linear.cu, csrc/layer_stack.cu), which choose that kernel themselves, are left out.
+USE_2SM = os.environ.get("PMETAL_GEMM_2SM", "1") == "1"
 # Reductions over tokens (LoRA dA / dB, weight gradients) are split across CTAs and summed with fp32 atomics, whose
 # order varies from run to run. With PMETAL_DETERMINISTIC=1 every output tile is owned by one CTA and accumulated in a
 # fixed order instead (slower for the skinny LoRA products, bitwise reproducible).
@@ -361,7 +363,7 @@ def _lora_call(name: str, spec: str, *args) -> None:
 def _lora_fused_ok(x, a, b, seg_sizes, r: int, *more) -> bool:
     """Whether a layer's narrow and wide products run from one call (csrc/lora_linear.cu): the rules of csrc/lora_tall.cu and of the GEMMs."""
     n = len(seg_sizes)
-    return (MN_MAJOR and not TUNA and not DETERMINISTIC and x.shape[0] > 128 and r % 8 == 0 and n * r <= 64 and n <= 4
+    return (MN_MAJOR and USE_2SM and not TUNA and not DETERMINISTIC and x.shape[0] > 128 and r % 8 == 0 and n * r <= 64 and n <= 4
             and all(s % 128 == 0 for s in seg_sizes[:-1]) and seg_sizes[-1] % 64 == 0 and x.shape[1] % 8 == 0 and a.shape[0] == n * r and b.shape[1] == r
             and a.is_contiguous() and b.is_contiguous() and (a.data_ptr() | b.data_ptr()) % 16 == 0
             and all(t.dtype == torch.bfloat16 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (x, *more)))
@@ -1038,6 +1040,10 @@ def _paged_route(meta, hq: int, hkv: int, int8: bool):
     if not int8 and _paged_on_tensor_cores(n_seq, meta.max_q, meta.max_kv, hq, hkv):
         return PAGED_TENSOR, 1
     return PAGED_SPLIT, _paged_splits(n_seq, meta.max_kv, hkv)
+
+
+def layer_stack_ok(tokens: int) -> bool:
+    return USE_2SM or tokens < 256
 
 
 def layer_stack(rows, x, meta, cos, sin, hq: int, hkv: int, inter: int, num_blocks: int, eps: float, scale: float):

@@ -73,3 +73,47 @@ def test_pair_gemm_into_a_wider_matrix(N):
     _near(out[:, :N], x.float() @ w.float().t() + wide[:, :N].float(), "result")
     assert bool((out[:, N:] == 7).all())
     nat.check_status()
+
+
+def test_the_pair_kernel_can_be_switched_off(monkeypatch):
+    """Without it neither a LoRA layer nor a prompt launches it, and the results stay."""
+    from pmetal_b200.models.config import ModelArgs
+    from pmetal_b200.models.decoder import DecoderLM
+    from pmetal_b200.models.generation import Generator
+    from pmetal_b200.ops import functional as ops
+    from pmetal_b200.ops import native as nat
+    g = torch.Generator(device="cuda").manual_seed(2)
+    f = lambda *s: torch.randn(*s, device="cuda", generator=g)      # noqa: E731
+    x, w, a, b = f(300, 256).bfloat16().requires_grad_(True), f(256, 256).bfloat16() / 16, f(16, 256) / 16, f(256, 16) / 4
+    a.requires_grad_(True), b.requires_grad_(True)
+    m = DecoderLM(ModelArgs(vocab_size=64, hidden_size=256, intermediate_size=256, num_hidden_layers=2, num_attention_heads=2,
+                            num_key_value_heads=1, head_dim=128)).init_weights(0.05, 1).to("cuda").to(torch.bfloat16).eval()
+    for p in m.parameters():
+        p.requires_grad_(False)
+
+    class Counting:
+        def __init__(self, real):
+            self.real, self.names = real, []
+
+        def __getattr__(self, name):
+            self.names.append(name)
+            return getattr(self.real, name)
+
+    def both():
+        counter = Counting(nat.lib())
+        with monkeypatch.context() as mp:
+            mp.setattr(nat, "lib", lambda: counter)
+            mp.setattr(nat, "_LORA_ARGS", {})
+            y = ops.lora_linear(x, w, None, a, b, (256,), 16, 1.0)
+            grads = torch.autograd.grad(y.float().square().sum(), (x, a, b))
+            gen = Generator(m, num_blocks=16, cuda_graphs=False)
+            out = [y, *grads, gen.prefill([gen.new_seq()], [list(range(60)) * 5])]
+        return [t.detach().float() for t in out], set(counter.names)
+    on, names = both()
+    assert names & {"pm_lora_linear_fwd", "pm_lora_linear_bwd", "pm_layer_stack"} == {"pm_lora_linear_fwd", "pm_lora_linear_bwd", "pm_layer_stack"}
+    monkeypatch.setattr(nat, "USE_2SM", False)
+    off, names = both()
+    assert not names & {"pm_lora_linear_fwd", "pm_lora_linear_bwd", "pm_layer_stack", "pm_gemm_bf16_2sm"}
+    for p, q in zip(on, off):
+        assert float((p - q).norm() / q.norm()) < 2e-2               # two layers of bf16 activations
+    nat.check_status()
