@@ -141,28 +141,32 @@ def test_grpo_step_on_gpu():
     native.check_status()
 
 
-def test_fp8_weights_and_speculative_and_engine():
+def _layer_by_layer(patch):
+    """Cached forwards go through the layers one by one inside the patch's context."""
+    from pmetal_b200.models.decoder import DecoderLM
+    patch.setattr(DecoderLM, "_stack_addresses", lambda self, cache: None)
+
+
+def test_fp8_weights_and_speculative_and_engine(monkeypatch):
     from pmetal_b200.models.fp8 import quantize_model_fp8
     from pmetal_b200.models.generation import Generator
     from pmetal_b200.models.sampling import SamplingParams
     from pmetal_b200.models.speculative import SpeculativeConfig, SpeculativeDecoder
     from pmetal_b200.ops import native
     from pmetal_b200.serve.engine import ContinuousBatchEngine, Request
-    from pmetal_b200.models import decoder
     target = _freeze(_small(layers=3))
     prompts = [torch.randint(0, 2048, (n,)).tolist() for n in (9, 70)]
-    # Exact agreement needs the draft step (one new token per row) and the verify step (five per row) to round the
-    # same way; the per-layer kernels do, the whole-step decode kernel sums in another order, so it is off here.
-    decoder.DECODE_MEGA = False
-    try:
+    # Exact agreement needs the draft step (one new token per row) and the verify step (five per row) to round the same way; the
+    # layer-by-layer path does at these sizes.
+    with monkeypatch.context() as patch:
+        _layer_by_layer(patch)
         base = Generator(target, num_blocks=128).generate(prompts, SamplingParams.greedy(20))
         # speculative decoding with the target as its own draft: same tokens, everything accepted
         sd = SpeculativeDecoder(target, target, SpeculativeConfig(num_draft_tokens=4, temperature=0.0, adaptive_k=False), 128, 128)
         out = sd.generate(prompts, 20)
         assert out == base.tokens and sd.stats.acceptance_rate > 0.99
-    finally:
-        decoder.DECODE_MEGA = True
-    # with the whole-step kernel drafting, the accepted text is still the target's own greedy continuation up to ties
+    # with all layers in one call, which sums in another order, the accepted text is that path's own greedy continuation up to ties
+    base = Generator(target, num_blocks=128).generate(prompts, SamplingParams.greedy(20))
     sd2 = SpeculativeDecoder(target, target, SpeculativeConfig(num_draft_tokens=4, temperature=0.0, adaptive_k=False), 128, 128)
     out2 = sd2.generate(prompts, 20)
     assert [o[:3] for o in out2] == [t[:3] for t in base.tokens] and sd2.stats.acceptance_rate > 0.5
@@ -249,10 +253,9 @@ def test_moe_training_step_runs_on_grouped_kernels_and_matches_reference():
 
 
 @pytest.mark.parametrize("batch,heads,kv_heads", [(1, 4, 2), (3, 4, 1), (9, 2, 2), (2, 4, 2)])
-def test_whole_step_decode_kernel_matches_per_layer_path(batch, heads, kv_heads):
-    """The single-launch decode step (all layers, grid barriers between phases) against the six-launches-per-layer
-    path on the same weights, cache contents and tokens."""
-    from pmetal_b200.models import decoder
+def test_whole_step_decode_kernel_matches_per_layer_path(batch, heads, kv_heads, monkeypatch):
+    """Decode steps with all layers in one call (norms inside the projections) against the layer-by-layer path on the same weights,
+    cache contents and tokens."""
     from pmetal_b200.models.config import ModelArgs
     from pmetal_b200.models.decoder import DecoderLM
     from pmetal_b200.models.generation import Generator
@@ -266,21 +269,23 @@ def test_whole_step_decode_kernel_matches_per_layer_path(batch, heads, kv_heads)
     g = torch.Generator().manual_seed(7)
     first = 650 if batch == 2 else 70          # the two-row case is long enough for several key splits per row
     prompts = [torch.randint(0, cfg.vocab_size, (first + 37 * i,), generator=g).tolist() for i in range(batch)]
-    outs = {}
-    for mega in (False, True):
-        decoder.DECODE_MEGA = mega
-        gen = Generator(m, num_blocks=64, cuda_graphs=False)
-        seqs = [gen.new_seq() for _ in prompts]
-        logits = gen.prefill(seqs, prompts)
-        ids = logits.argmax(-1)
-        trace = []
-        for _ in range(4):
-            logits = gen.decode_step(seqs, ids)
-            trace.append(logits.float().clone())
-            ids = logits.argmax(-1)
-        outs[mega] = torch.stack(trace)
+    outs, calls = {}, []
+    monkeypatch.setattr(native, "layer_stack", lambda *a, _f=native.layer_stack: calls.append(1) or _f(*a))
+    fed = None
+    for one_call in (False, True):
+        with monkeypatch.context() as patch:
+            if not one_call:
+                _layer_by_layer(patch)
+            gen = Generator(m, num_blocks=64, cuda_graphs=False)
+            seqs = [gen.new_seq() for _ in prompts]
+            steps = [gen.prefill(seqs, prompts)]
+            for k in range(4):
+                # both sides are fed what the first one chose: a tie that falls the other way is no disagreement
+                steps.append(gen.decode_step(seqs, fed[k] if one_call else steps[-1].argmax(-1)))
+        fed = fed or [x.argmax(-1) for x in steps]
+        outs[one_call] = torch.stack([x.float() for x in steps[1:]])
+        assert len(calls) == (5 if one_call else 0)
         native.check_status()
-    decoder.DECODE_MEGA = True
     a, b = outs[False], outs[True]
     assert torch.isfinite(b).all()
     err = (a - b).abs().max().item()
@@ -312,17 +317,17 @@ def test_decode_with_4bit_base_weights_uses_the_fused_kernel():
         fp.weight.data.copy_(dequantize(fq.qweight, torch.bfloat16))
         assert fq.gemv_ok(1) and fq.weight.numel() == 0
     prompts = [torch.randint(0, 512, (40,)).tolist(), torch.randint(0, 512, (75,)).tolist()]
-    outs = []
+    outs, fed = [], None
     for m in (packed, plain):
         gen = Generator(m, num_blocks=32, cuda_graphs=False)
         seqs = [gen.new_seq() for _ in prompts]
-        ids = gen.prefill(seqs, prompts).argmax(-1)
-        steps = []
-        for _ in range(3):
-            logits = gen.decode_step(seqs, ids)
-            steps.append(logits.float())
-            ids = logits.argmax(-1)
-        outs.append(torch.stack(steps))
+        steps = [gen.prefill(seqs, prompts)]
+        for k in range(3):
+            # both models are fed what the first one chose: their prompts round differently (0.03 of logits up to 3), and in 2 % of rows
+            # a tie falls the other way
+            steps.append(gen.decode_step(seqs, fed[k] if fed else steps[-1].argmax(-1)))
+        fed = fed or [x.argmax(-1) for x in steps]
+        outs.append(torch.stack([x.float() for x in steps[1:]]))
         native.check_status()
     a, b = outs
     assert torch.isfinite(a).all()
