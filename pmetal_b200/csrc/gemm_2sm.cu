@@ -421,6 +421,7 @@ extern "C" int pm_gemm_bf16_2sm(const void* A, int a_mn, int lda, int a_rows, co
   if (tail && (out_mode != 0 || R || tail_from % 8 || (reinterpret_cast<uintptr_t>(tail) & 15))) return -20;
   if (splits < 1 || (splits > 1 && (out_mode < 2 || out_mode > 3))) return -12;   // split-K needs the atomic modes
   if (M <= 0 || N <= 0 || K <= 0) return -13;
+  if (seg_mode < 0 || seg_mode > 2) return -16;
   if (out_mode == 0 && ((ldd % 8) || (reinterpret_cast<uintptr_t>(D) & 15))) return -14;
   if (R && ((ldr % 8) || (reinterpret_cast<uintptr_t>(R) & 15))) return -15;
   GemmParams p{};

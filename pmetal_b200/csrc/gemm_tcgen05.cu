@@ -282,6 +282,7 @@ extern "C" int pm_gemm_bf16(const void* A, int a_mn, int lda, int a_rows, const 
     if (static_cast<long long>(splits - 1) * per >= nk_all) return -18;
   }
   if (M <= 0 || N <= 0 || K <= 0) return -13;
+  if (seg_mode < 0 || seg_mode > 2) return -16;
   if ((out_mode == 0 || out_mode == 6) && ((ldd % 8) || (reinterpret_cast<uintptr_t>(D) & 15))) return -14;
   if (R && ((ldr % 8) || (reinterpret_cast<uintptr_t>(R) & 15))) return -15;
   GemmParams p{};

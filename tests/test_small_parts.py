@@ -149,3 +149,19 @@ def test_steps_of_a_few_tokens_take_the_faster_attention_kernel(int8, n, ctx, q,
     from pmetal_b200.ops import native
     meta = BatchMeta(list(range(n)), torch.zeros(n, ctx // 64 + 1, dtype=torch.int32), None, None, None, None, None, n * q, q, ctx)
     assert (native._paged_route(meta, hq, hkv, bool(int8))[0] == native.PAGED_DECODE) == apart
+
+
+@pytest.mark.parametrize("name", ["pm_gemm_bf16", "pm_gemm_bf16_2sm"])
+def test_gemm_entries_refuse_segment_modes_that_they_do_not_have(name):
+    """Mode 3 (segments of the reduction) belongs to pm_lora_tall; a GEMM that took it for no segments would answer wrongly."""
+    from pmetal_b200.ops import native
+    if native.load_error():
+        pytest.skip(native.load_error())
+    i, p, ll = native.c_int, native._p(None), native.c_ll
+    one = [i(64)]                                                                   # bn: the pair kernel chooses its own
+    head = [p, i(0), i(64), i(64), p, i(0), i(64), i(64), p, i(0), i(0), i(0), p, i(0), i(0), i(0), p, i(0), i(64), p, i(0), i(64), i(64), i(64), i(0),
+            i(0), native.c_float(1.0)]
+    tail = [i(1), i(3), None, i(16), i(0)]
+    end = [p, i(0), i(0), p, native.c_void_p(0)]
+    args = head + tail + end if name.endswith("2sm") else head + one + tail + [p, ll(0), p, ll(0)] + end
+    assert getattr(native.lib(), name)(*args) == -16
