@@ -44,14 +44,9 @@ __device__ __forceinline__ float row_max(uint32_t taddr, int lo, int span) {
   return mx;
 }
 
-// p = exp2(s * a + b) for the 128 columns of this row, written as bf16 into the swizzled P tile; returns the row sum. Capped:
-// p = exp2(b - c / (exp2(s * a) + 1)), a capped score in base 2 when c is twice the cap and b contains the cap
-// (tanh(x) = 1 - 2 / (exp(2 x) + 1)). Sigmoid weights: p = 1 / (1 + exp2(s * a + b)).
-enum : int { kFaPlain = 0, kFaCapped = 1, kFaSigmoid = 2 };
-
-template <bool kMask, int kMode>
-__device__ __forceinline__ float exp_rows(uint32_t taddr, uint32_t tile_addr, int r, float a, float b, int lo,
-                                          int span, float c2 = 0.f) {
+// p = exp2(s * a + b) for the 128 columns of this row, written as bf16 into the swizzled P tile; returns the row sum.
+template <bool kMask>
+__device__ __forceinline__ float exp_rows(uint32_t taddr, uint32_t tile_addr, int r, float a, float b, int lo, int span) {
   float rs = 0.f;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
@@ -61,17 +56,7 @@ __device__ __forceinline__ float exp_rows(uint32_t taddr, uint32_t tile_addr, in
     uint32_t pk[16];
 #pragma unroll
     for (int e = 0; e < 32; e += 2) {
-      float p0, p1;
-      if (kMode == kFaSigmoid) {
-        p0 = fast_rcp(1.f + fast_exp2(fmaf(__uint_as_float(v[e]), a, b)));
-        p1 = fast_rcp(1.f + fast_exp2(fmaf(__uint_as_float(v[e + 1]), a, b)));
-      } else if (kMode == kFaCapped) {
-        p0 = fast_exp2(fmaf(-c2, fast_rcp(fast_exp2(__uint_as_float(v[e]) * a) + 1.f), b));
-        p1 = fast_exp2(fmaf(-c2, fast_rcp(fast_exp2(__uint_as_float(v[e + 1]) * a) + 1.f), b));
-      } else {
-        p0 = fast_exp2(fmaf(__uint_as_float(v[e]), a, b));
-        p1 = fast_exp2(fmaf(__uint_as_float(v[e + 1]), a, b));
-      }
+      float p0 = fast_exp2(fmaf(__uint_as_float(v[e]), a, b)), p1 = fast_exp2(fmaf(__uint_as_float(v[e + 1]), a, b));
       if (kMask) {
         const bool any = span >= 0;
         p0 = (any && static_cast<unsigned>(c * 32 + e - lo) <= static_cast<unsigned>(span)) ? p0 : 0.f;
@@ -240,8 +225,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         break;
       }
       // pass 2: p = exp2(s * scale - m), row sum, bf16 P into shared memory (128B-swizzled, two 64-key boxes)
-      const float rs = need_mask ? exp_rows<true, kFaPlain>(tmem_base + b * 128 + lane_off, sP_addr, r, sl2, -m_use, lo, span)
-                                 : exp_rows<false, kFaPlain>(tmem_base + b * 128 + lane_off, sP_addr, r, sl2, -m_use, 0, 0);
+      const float rs = need_mask ? exp_rows<true>(tmem_base + b * 128 + lane_off, sP_addr, r, sl2, -m_use, lo, span)
+                                 : exp_rows<false>(tmem_base + b * 128 + lane_off, sP_addr, r, sl2, -m_use, 0, 0);
       l_run = l_run * corr + rs;
       fence_async_smem();        // generic-proxy writes of P -> visible to the tensor-core (async) proxy
       tc_fence_before();         // this thread's TMEM reads of S are complete
@@ -374,7 +359,10 @@ __device__ __forceinline__ float fa_row_max(const float (&x)[128], int lo, int s
     m[e & 3] = fmaxf(m[e & 3], !kMask || static_cast<unsigned>(e - from) <= last ? x[e] : -INFINITY);
   return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
 }
-// exp_rows for a row that is in registers; the sum runs in four independent chains.
+// exp_rows for a row that is in registers; the sum runs in four independent chains. Capped: p = exp2(b - c / (exp2(s * a) + 1)), a capped
+// score in base 2 when c is twice the cap and b contains the cap (tanh(x) = 1 - 2 / (exp(2 x) + 1)). Sigmoid weights:
+// p = 1 / (1 + exp2(s * a + b)).
+enum : int { kFaPlain = 0, kFaCapped = 1, kFaSigmoid = 2 };
 template <bool kMask, int kMode>
 __device__ __forceinline__ float fa_exp_row(const float (&x)[128], uint32_t tile_addr, int r, float a, float b, int lo, int span,
                                             float c2) {

@@ -30,6 +30,22 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t ran
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
   return r;
 }
+// reads of another CTA's shared memory at an address that map_to_cta gave
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -51,22 +67,14 @@ __device__ __forceinline__ void tma_load_2d_local(uint32_t dst_smem, const CUten
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_addr), "r"(c0), "r"(c1)
       : "memory");
 }
-template <bool kLocal>
-__device__ __forceinline__ void load_operand_pair_t(uint32_t dst, const CUtensorMap* map, uint32_t bar, int mn_major,
-                                                    int rows, int row0, int k0) {
+// One operand tile of the 4-bit kernel: bytes are counted on this CTA's own barrier.
+__device__ __forceinline__ void load_operand_local(uint32_t dst, const CUtensorMap* map, uint32_t bar, int mn_major, int rows, int row0,
+                                                   int k0) {
   if (!mn_major) {
-    if (kLocal) tma_load_2d_local(dst, map, bar, k0, row0); else tma_load_2d_pair(dst, map, bar, k0, row0);
+    tma_load_2d_local(dst, map, bar, k0, row0);
   } else {
-    for (int j = 0; j < rows / 64; ++j) {
-      if (kLocal) tma_load_2d_local(dst + j * 8192, map, bar, row0 + 64 * j, k0);
-      else tma_load_2d_pair(dst + j * 8192, map, bar, row0 + 64 * j, k0);
-    }
+    for (int j = 0; j < rows / 64; ++j) tma_load_2d_local(dst + j * 8192, map, bar, row0 + 64 * j, k0);
   }
-}
-__device__ __forceinline__ void load_operand_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int mn_major,
-                                                  int rows, int row0, int k0, int local) {
-  if (local) load_operand_pair_t<true>(dst, map, bar, mn_major, rows, row0, k0);
-  else load_operand_pair_t<false>(dst, map, bar, mn_major, rows, row0, k0);
 }
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
   uint32_t ok;

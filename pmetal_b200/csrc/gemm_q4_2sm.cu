@@ -160,15 +160,15 @@ gemm_q4_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           const uint32_t fb = smem_u32(&full_bar[s]);
           if (kb < p.nk1) {
             mbar_expect_tx(&full_bar[s], a_bytes);
-            load_operand_pair_t<true>(sa, &map_a, fb, 0, kBM, m0, kb * kBK);
+            load_operand_local(sa, &map_a, fb, 0, kBM, m0, kb * kBK);
             mbar_expect_tx(&cfull_bar[s], kQ4CodeBytes);
             if (!q.trans) tma_load_2d_local(sc, &map_c, smem_u32(&cfull_bar[s]), kb * (kBK / 2), n0);
             else tma_load_2d_local(sc, &map_c, smem_u32(&cfull_bar[s]), n0 / 2, kb * kBK);
           } else {
             const int k0 = (kb - p.nk1) * kBK;
             mbar_expect_tx(&full_bar[s], a_bytes + b_bytes);
-            load_operand_pair_t<true>(sa, &map_a2, fb, p.a2_mn, kBM, m0, k0 + a2_off);
-            load_operand_pair_t<true>(sb, &map_b2, fb, p.b2_mn, kHalfBN, n0, k0);
+            load_operand_local(sa, &map_a2, fb, p.a2_mn, kBM, m0, k0 + a2_off);
+            load_operand_local(sb, &map_b2, fb, p.b2_mn, kHalfBN, n0, k0);
             mbar_arrive(&cfull_bar[s]);         // nothing to expand in this block
           }
         }

@@ -20,7 +20,7 @@
 
 namespace pm {
 
-struct SkinnyParams {
+struct FewRowParams {
   __nv_bfloat16* y;
   const __nv_bfloat16* res;
   long long ldy, ldr;
@@ -41,21 +41,10 @@ struct SkinnyParams {
 
 constexpr int kSkW = 128 * 64 * 2;        // one k block of a weight tile: 16 KB
 
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
-  return v;
-}
-
 // Sum over the cluster and epilogue of this CTA's share of the token rows, one warp per row; all loads of a row are in flight
 // together. Ends with this thread's arrival at the cluster barrier behind which the partial tiles may go away.
 template <int kSplits>
-__device__ __forceinline__ void skinny_finish(const SkinnyParams& p, uint32_t part, int split, int n0, const float* s_rstd) {
+__device__ __forceinline__ void skinny_finish(const FewRowParams& p, uint32_t part, int split, int n0, const float* s_rstd) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t at[kSplits];
 #pragma unroll
@@ -125,7 +114,7 @@ __device__ __forceinline__ void skinny_finish(const SkinnyParams& p, uint32_t pa
 // [kMT][128] once the MMAs are done.
 template <int kMT>
 __global__ void __launch_bounds__(kThreads)
-skinny_linear_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SkinnyParams p) {
+skinny_linear_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const FewRowParams p) {
   constexpr int kStage = kSkW + kMT * 128;
   constexpr int kCols = kMT < 32 ? 32 : kMT;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -292,7 +281,7 @@ __global__ void __launch_bounds__(256) skinny_prep_kernel(const __nv_bfloat16* _
 }
 
 template <int kMT>
-static int launch_skinny(const CUtensorMap& mw, const CUtensorMap& mx, SkinnyParams p, int tiles, int chain, cudaStream_t st) {
+static int launch_skinny(const CUtensorMap& mw, const CUtensorMap& mx, FewRowParams p, int tiles, int chain, cudaStream_t st) {
   constexpr int kStage = kSkW + kMT * 128;
   // two CTAs to an SM, so that the next kernel of a chain can move in: about 100 KB each
   p.stages = std::min(std::min(kMaxStages, 100 * 1024 / kStage), std::max(p.per, 1));
@@ -343,7 +332,7 @@ extern "C" int pm_linear_skinny_norm(const void* x, long long ldx, const void* w
        reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(y2) | reinterpret_cast<uintptr_t>(nw_out)) & 15)
     return -3;
   if (y2 && (swiglu || !nw_out || !ss_out)) return -5;
-  SkinnyParams p{};
+  FewRowParams p{};
   p.y = static_cast<__nv_bfloat16*>(y); p.ldy = ldy;
   p.res = static_cast<const __nv_bfloat16*>(res); p.ldr = ldr;
   p.M = M; p.N = N; p.K = K; p.swiglu = swiglu; p.alpha = alpha; p.status = status;

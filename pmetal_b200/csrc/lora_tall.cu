@@ -26,12 +26,6 @@ struct TallParams {
 constexpr int kTlStage = 128 * 128 + 64 * 128;      // X [128][64], B [64][64]
 constexpr int kTlLd = 68;                           // floats per row of the partial tile: 16-byte rows on different banks
 
-__device__ __forceinline__ float4 tl_ld_cluster(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-  return v;
-}
-
 template <int kSplits>
 __device__ __forceinline__ void tall_finish(const TallParams& p, uint32_t part, int split, int m0) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = (lane & 15) * 4;
@@ -43,7 +37,7 @@ __device__ __forceinline__ void tall_finish(const TallParams& p, uint32_t part, 
     const int row = split * kShare + r;
     float4 v[kSplits];
 #pragma unroll
-    for (int i = 0; i < kSplits; ++i) v[i] = tl_ld_cluster(at[i] + (row * kTlLd + c) * 4);
+    for (int i = 0; i < kSplits; ++i) v[i] = ld_cluster_f4(at[i] + (row * kTlLd + c) * 4);
     float f[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < kSplits; ++i) { f[0] += v[i].x; f[1] += v[i].y; f[2] += v[i].z; f[3] += v[i].w; }

@@ -69,12 +69,6 @@ __device__ __forceinline__ uint32_t pd_rest(float a, float b, uint32_t packed) {
 __device__ __forceinline__ uint32_t pd_code(uint32_t biased, int i) {
   return __float_as_uint(__uint_as_float(__byte_perm(biased, 0x4B000000u, 0x7540u | i)) - 8388736.f);
 }
-__device__ __forceinline__ float pd_ld_cluster(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-
 // 16 bytes of row `row` (128 bytes, 128B-swizzled box) of a stage
 __device__ __forceinline__ uint4 pd_lds16(uint32_t box, int row, int chunk) {
   uint4 v;
@@ -392,9 +386,9 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       lv[c] = ov[c] = 0.f;
       if (c < p.splits) {
         const uint32_t ml = map_to_cta(ml_addr, c) + h * 8;
-        mv[c] = pd_ld_cluster(ml);
-        lv[c] = pd_ld_cluster(ml + 4);
-        ov[c] = pd_ld_cluster(map_to_cta(o_addr, c) + e * 4);
+        mv[c] = ld_cluster_f32(ml);
+        lv[c] = ld_cluster_f32(ml + 4);
+        ov[c] = ld_cluster_f32(map_to_cta(o_addr, c) + e * 4);
       }
     }
 #pragma unroll

@@ -2,8 +2,9 @@
 // attribute may start while its predecessor in the stream is still running. Everything it does before pdl_wait() must
 // be independent of the predecessor's output (reading weights, prefetching them into L2); pdl_wait() returns once the
 // predecessor has completed and its writes are visible. Every kernel of a chain calls pdl_launch_dependents() at its
-// top so that its successor can be scheduled as soon as all of this kernel's CTAs are resident. Both instructions are
-// no-ops in a kernel launched the ordinary way. launch_pdl sets the launch attribute inside a PdlScope (the chains of
+// top so that its successor can be scheduled as soon as all of this kernel's CTAs are resident. In a kernel launched the ordinary way
+// only pdl_wait() is a no-op: its pdl_launch_dependents() still lets an attributed successor start early. What a kernel reads before
+// pdl_wait() must therefore be older than the whole chain, attributed or not. launch_pdl sets the launch attribute inside a PdlScope (the chains of
 // layer_stack.cu) or with PMETAL_PDL=1.
 #pragma once
 #include <cuda_runtime.h>

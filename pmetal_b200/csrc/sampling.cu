@@ -51,12 +51,6 @@ struct SampleParams {
   int ctas;                  // CTAs per row
 };
 
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-
 __device__ __forceinline__ uint32_t order_key(float f) {   // larger float -> larger key
   const uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);

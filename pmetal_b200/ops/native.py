@@ -495,7 +495,7 @@ def _splits_for(m_tiles: int, nk: int) -> int:
 
     Every (tile, split) pair is one CTA and an SM streams its operands at a fixed rate, so the launch takes
     waves * (k-blocks per split + a fixed cost per CTA) with waves = ceil(pairs / SMs). One pair more than there are SMs
-    doubles the time, so the count is chosen by that makespan, not by rounding SMs / tiles up."""
+    doubles the time, so the count is chosen by that makespan, not by rounding SMs / tiles up. csrc/lora_linear.cu has the same rule."""
     sms, m_tiles = sm_count(), max(m_tiles, 1)
     best, best_cost = 1, None
     for s in range(1, min(nk, 64) + 1):
