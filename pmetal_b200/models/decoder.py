@@ -35,11 +35,6 @@ ALL_PROJ = ATTN_PROJ + MLP_PROJ
 GEMV_MAX_ROWS = int(os.environ.get("PMETAL_GEMV_MAX_ROWS", "16"))
 
 
-def _call_is_wrapped(own: Dict) -> bool:
-    """Whether calling the module with this ``__dict__`` runs more than its class's ``forward``."""
-    return bool(own["_forward_hooks"] or own["_forward_pre_hooks"]) or "forward" in own
-
-
 class FusedLinear(nn.Module):
     """A row-stacked group of projections sharing one input, with optional LoRA.
 
@@ -529,28 +524,30 @@ class DecoderLM(nn.Module):
         for li, layer in enumerate(self.layers):
             mods = layer._modules
             at, mlp = mods["self_attn"], mods["mlp"]
-            if at.window or type(mlp) is not MLP or _call_is_wrapped(mlp.__dict__):
+            own = mlp.__dict__
+            if at.window or type(mlp) is not MLP or own["_forward_hooks"] or own["_forward_pre_hooks"] or "forward" in own:
                 return None
             w = []
             for lin in (at._modules["qkv_proj"], at._modules["o_proj"], mlp._modules["gate_up_proj"], mlp._modules["down_proj"]):
                 own = lin.__dict__
                 par = own["_parameters"]
                 p = par.get("weight")
-                if (p is None or type(lin) is not FusedLinear or _call_is_wrapped(own) or par.get("bias") is not None
-                        or par.get("lora_a") is not None or own.get("lora_a") is not None or own.get("qweight") is not None
-                        or (own.get("batched") is not None and own.get("adapter_rows") is not None)
-                        or p.requires_grad or p.dtype != dt or p.dim() != 2 or not p.is_contiguous() or p.data_ptr() % 16):
+                if (p is None or type(lin) is not FusedLinear or own["_forward_hooks"] or own["_forward_pre_hooks"] or "forward" in own
+                        or par.get("bias") is not None or par.get("lora_a") is not None or own.get("lora_a") is not None
+                        or own.get("qweight") is not None or (own.get("batched") is not None and own.get("adapter_rows") is not None)
+                        or p.requires_grad or p.dtype is not dt or p.dim() != 2 or not p.is_contiguous()):
                     return None
                 w.append(p.data_ptr())
             norms = layer._parameters["input_layernorm"], layer._parameters["post_attention_layernorm"]
             qk = (at._parameters["q_norm"], at._parameters["k_norm"]) if at.q_norm is not None else ()
-            if any(p.dtype != dt or p.data_ptr() % 16 for p in norms + qk):
-                return None
-            qn, kn = (p.data_ptr() for p in qk) if qk else (0, 0)
+            for p in norms + qk:
+                if p.dtype is not dt:
+                    return None
+            qn, kn = (qk[0].data_ptr(), qk[1].data_ptr()) if qk else (0, 0)
             rows += [norms[0].data_ptr(), w[0], qn, kn, w[1], norms[1].data_ptr(), w[2], w[3], cache.k[li].data_ptr(),
                      cache.v[li].data_ptr(), cache.k_scale[li].data_ptr() if cache.quant else 0,
                      cache.v_scale[li].data_ptr() if cache.quant else 0]
-        return rows
+        return None if any(a % 16 for a in rows) else rows
 
     def _paged_attention_reference(self, qkv, at, rope, cache, meta, li, hq=None, hkv=None):
         from ..ops import reference as ref

@@ -1014,7 +1014,7 @@ def _paged_tokens_apart(n_seq: int, max_q: int, max_kv: int, hkv: int, table: in
     16 x 700, 2 tokens 13.7, 15.7, 4 tokens 24.8, 15.8; 64 x 450, 2 tokens 32.6, 30.8, 8 tokens 86.1, 31.9; 8 x 6000, 2 tokens 45.4, 42.3;
     int8: 2 tokens 59.7, 69.4, 3 tokens 109.5, 69.5."""
     sms, blocks = sm_count(), -(-max_kv // 64)
-    ctas, splits = n_seq * max_q * hkv, 1
+    ctas, splits = max(n_seq * max_q * hkv, 1), 1
     while splits < 8 and ctas * splits * 2 <= 2 * sms and splits * 2 <= max(table, 8):      # as pm_paged_decode does
         splits *= 2
     ctas *= splits
